@@ -309,3 +309,137 @@ def tolerance(case):
     if case.get("rms"):
         return {"rel": 4e-3, "max": 6e-2, "differ": 1e-3}
     return {"rel": 3e-4, "max": 3.2e-2}
+
+
+# ---- the same results in 64 bits ---------------------------------------------------------------------
+
+def _e4m3(x, scale):
+    """x (fp32) in units of scale, rounded to e4m3: the rule of the FP8 quantizers, whose quotient is the IEEE fp32 one."""
+    return (x / scale).clamp(-448.0, 448.0).to(torch.float8_e4m3fn).float()
+
+
+def _fp8_scale(amax):
+    return (amax / torch.full_like(amax, 448.0)).clamp(min=1e-10)
+
+
+def _exact_rows(x):
+    x = x.float()
+    scale = _fp8_scale(x.abs().amax(1, keepdim=True))
+    return _e4m3(x, scale).double() * scale.double(), scale
+
+
+def _exact_1x128(x, norm=None):
+    x = x.double()
+    if norm is not None:
+        x = x * (x.square().mean(1, keepdim=True) + EPS).rsqrt() * norm.double()
+    g = x.float().view(x.shape[0], -1, 128)
+    scale = _fp8_scale(g.abs().amax(2, keepdim=True))
+    return (_e4m3(g, scale).double() * scale.double()).view_as(x), scale.squeeze(2)
+
+
+def _exact_128x128(w):
+    N, K = w.shape
+    t = w.float().view(N // 128, 128, K // 128, 128)
+    scale = _fp8_scale(t.abs().amax((1, 3), keepdim=True))
+    return (_e4m3(t, scale).double() * scale.double()).view(N, K)
+
+
+def _exact_mxfp4(x):
+    """Nearest e2m1 magnitude in units of 2^(floor(log2 amax) - 2) per 32 values; a tie goes to the smaller one."""
+    g = x.double().view(x.shape[0], -1, 32)
+    amax = g.abs().amax(2, keepdim=True)
+    e = torch.where(amax > 0, torch.frexp(amax).exponent - 3, -127).clamp(-127, 127)
+    unit = torch.ldexp(torch.ones_like(amax), e)
+    magnitudes = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device=DEV)
+    middles = torch.tensor([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0], dtype=torch.float64, device=DEV)
+    q = g / unit
+    return (magnitudes[torch.bucketize(q.abs(), middles)] * q.sign() * unit).view(x.shape)
+
+
+def _exact_pts(c, g):
+    B, M, N, K = c["batch"], c["M"], c["N"], c["K"]
+    x, xs = _exact_rows(_activations(g, B * M, K))
+    w, _ = _exact_rows(_weights(g, B * N, K))
+    y = x.view(B, M, K) @ w.view(B, N, K).mT
+    if c["bias"]:
+        y += torch.randn(B, N, generator=g, device=DEV).bfloat16().double()[:, None]
+    return (y[0] if B == 1 else y), None, xs
+
+
+def _exact_blockscale(c, g):
+    M, N, K = c["M"], c["N"], c["K"]
+    x = _activations(g, M, K)
+    w = _exact_128x128(_weights(g, N, K))
+    norm = (1.0 + 0.1 * torch.randn(K, generator=g, device=DEV)).bfloat16() if c["rms"] else None
+    x, xs = _exact_1x128(x, norm)
+    y = x @ w.T
+    if c["mul_add"]:
+        c_a, c_b = torch.randn(2, M, N, generator=g, device=DEV).bfloat16().unbind(0)
+        y = y * c_a + c_b
+    return y, None, xs
+
+
+def _exact_mxfp4_layer(c, g):
+    M, N, K = c["M"], c["N"], c["K"]
+    x = _exact_mxfp4(_activations(g, M, K))
+    y = x @ _exact_mxfp4(_weights(g, N, K)).T
+    if c["mul_add"]:
+        c_a, c_b = torch.randn(2, M, N, generator=g, device=DEV).bfloat16().unbind(0)
+        y = y * c_a + c_b
+    return y, None, None
+
+
+def _exact_ptgq(c, g):
+    B, M, N, K = c["batch"], c["M"], c["N"], c["K"]
+    w = _weights(g, B * N, K)
+    x = _activations(g, B * M, K).float().view(B, M, K // 64, 64)
+    ws = (w.abs().max().float() / 448.0).reshape(1)
+    w = _e4m3(w.float(), ws).double().view(B, N, K) * ws.double()
+    scale = x.abs().amax(3, keepdim=True).clamp(min=1e-10) * (1.0 / 448.0)
+    x = (x * scale.reciprocal()).to(torch.float8_e4m3fn).float().double() * scale.double()
+    y = x.view(B, M, K) @ w.mT
+    if c["bias"]:
+        y += torch.randn(B, 1, N, generator=g, device=DEV).bfloat16().double()
+    return y
+
+
+def _exact_moe_fp8(c, g):
+    T, E, N, K, k = c["tokens"], c["experts"], c["N"], c["K"], c["top_k"]
+    _, order, hist = _routing(g, T, E, k)
+    x, xs = _exact_1x128(_activations(g, T, K))
+    y = _empty(T * k, N, dtype=torch.float64)
+    at = 0
+    for n in hist:
+        w = _exact_128x128(_weights(g, N, K))
+        torch.matmul(x[order[at: at + n].long() // k], w.T, out=y[at: at + n])
+        at += n
+    if c["bias"]:
+        y += torch.randn(E, N, generator=g, device=DEV).double().repeat_interleave(torch.tensor(hist, device=DEV), 0)
+    return y, None, xs
+
+
+def _exact_moe_mxfp4(c, g):
+    T, E, N, K, k = c["tokens"], c["experts"], c["N"], c["K"], c["top_k"]
+    _, order, hist = _routing(g, T, E, k)
+    x = _exact_mxfp4(_activations(g, T, K))
+    gate = torch.rand(T * k, generator=g, device=DEV).double()
+    y = _empty(T * k, N, dtype=torch.float64)
+    at = 0
+    for n in hist:
+        w = _exact_mxfp4(_weights(g, N, K))
+        ids = order[at: at + n].long()
+        y[ids] = (x[ids // k] @ w.T) * gate[ids, None]
+        at += n
+    return y, None, None
+
+
+_EXACT = {"pts": _exact_pts, "blockscale": _exact_blockscale, "mxfp4": _exact_mxfp4_layer, "ptgq": _exact_ptgq, "moe_fp8": _exact_moe_fp8,
+          "moe_mxfp4": _exact_moe_mxfp4}
+
+
+def exact(case, seed):
+    """What `run` returns, as plain torch gives it: the operands that the rules of the quantizers define, their products in 64 bits.
+    None in the place of codes, and for a case of over 1e14 operations."""
+    if work(case)["flops"] > 1e14:
+        return None
+    return _EXACT[case["kind"]](case, _gen(seed))

@@ -1,0 +1,25 @@
+"""GPU tier: the edges of single kernels and of the dispatch rules between them, against the oracle or an exact restatement."""
+import pytest
+import torch
+
+from test_gemm_gpu import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+def _tc_layout(sf, batch, rows, K):
+    """Row-major e8m0 bytes -> 512-byte atoms (128 rows x 4 bytes, byte (r % 32) * 16 + (r // 32) * 4 + j), zero-padded."""
+    katoms, rblks = (K // 128 + 1) & ~1, 2 * ((rows + 255) // 256) + 2
+    full = torch.zeros(batch, rblks * 128, katoms * 4, dtype=torch.uint8, device=sf.device)
+    full[:, :rows, : K // 32] = sf.view(batch, rows, K // 32)
+    return full.view(batch, rblks, 4, 32, katoms, 4).permute(0, 1, 4, 3, 2, 5).reshape(-1)
+
+
+@pytest.mark.parametrize("batch,rows,K", [(1, 1, 128), (1, 129, 384), (3, 200, 640), (1, 255, 1024), (2, 128, 1152), (1, 3080, 4224)])
+def test_mxfp4_scale_prepass_layout(hk, batch, rows, K):
+    """Whole and ragged 128-row blocks, 8-atom chunks and 16-byte row pieces: every byte of the layout."""
+    sf = torch.randint(1, 255, (batch * rows, K // 32), generator=torch.Generator().manual_seed(rows), dtype=torch.uint8).to(DEV)
+    mod = hk.gemm.afp4wfp4
+    out = torch.full((mod.sf_tc_bytes(batch, rows, K),), 0xEE, dtype=torch.uint8, device=DEV)
+    mod.sf_to_tc(sf if batch == 1 else sf.view(batch, rows, K // 32), out, K)
+    assert torch.equal(out, _tc_layout(sf, batch, rows, K))

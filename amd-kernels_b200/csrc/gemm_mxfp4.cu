@@ -163,6 +163,43 @@ struct Cfg {
     static_assert(kDynamic <= 232448, "shared memory budget");
 };
 
+// c_a / c_b of 32 consecutive columns of one row, for the fused multiply-add epilogue.  All eight 16-byte loads of a
+// chunk go out together, one chunk ahead of its use (the first before the accumulator is waited for), behind an L2
+// prefetch of the tile's whole row: loaded where they were used, four round trips to HBM per chunk one after the other,
+// they took more of a tile's time than its main loop (M = 1000, N = 3080, K = 4224: 34.5 us before, 21.4 now with the same 128-wide tiles).
+struct MulAddChunk {
+    uint4 a[4], b[4];
+    __device__ __forceinline__ void fetch(const Mxfp4Params& p, int64_t row_off, int col0, bool row_ok) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const bool in = row_ok && col0 + 8 * j < p.N;
+            a[j] = in ? __ldg(reinterpret_cast<const uint4*>(p.c_a + row_off + col0 + 8 * j)) : make_uint4(0, 0, 0, 0);
+            b[j] = in ? __ldg(reinterpret_cast<const uint4*>(p.c_b + row_off + col0 + 8 * j)) : make_uint4(0, 0, 0, 0);
+        }
+    }
+    __device__ __forceinline__ void apply(uint32_t (&r)[32]) const {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float ca[8], cb[8];
+            unpack8(a[j], ca);
+            unpack8(b[j], cb);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[8 * j + i] = __float_as_uint(__fmaf_rn(ca[i], __uint_as_float(r[8 * j + i]), cb[i]));
+        }
+    }
+};
+// The tile's part of one row of c_a and c_b into L2: one prefetch per 128 bytes of the BN columns from col0.
+template <int BN>
+__device__ __forceinline__ void prefetch_mul_add(const Mxfp4Params& p, int64_t row_off, int col0, bool row_ok) {
+    if (!row_ok) return;
+#pragma unroll
+    for (int c = 0; c < BN; c += 64)
+        if (col0 + c < p.N) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.c_a + row_off + col0 + c));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.c_b + row_off + col0 + c));
+        }
+}
+
 template <int BN>
 __global__ void __launch_bounds__(192, 1)
 gemm_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Mxfp4Params p) {
@@ -326,6 +363,11 @@ gemm_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             }
             const int64_t row_off = ((int64_t)b * p.M + (row_ok ? row : 0)) * p.N;
             __nv_bfloat16* crow = p.C + row_off;
+            MulAddChunk ma;
+            if (p.c_a) {
+                prefetch_mul_add<BN>(p, row_off, nb * BN, row_ok);
+                ma.fetch(p, row_off, nb * BN, row_ok);
+            }
             if (!__all_sync(0xFFFFFFFFu, mbar_wait(tfull_bar(acc), acc_ph, abort_flag, p.status, kErrWaitEpilogue))) break;
             tc_fence_after();
             const uint32_t t_addr = tmem_base + lane_addr + acc * BN;
@@ -334,18 +376,15 @@ gemm_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 uint32_t r[32];
                 tmem_ld32(t_addr + c, r);
                 tmem_ld_wait();
+                if (p.c_a) {
+                    ma.apply(r);
+                    if (c + 32 < BN) ma.fetch(p, row_off, nb * BN + c + 32, row_ok);
+                }
                 if (row_ok) {
                     const int col0 = nb * BN + c;
 #pragma unroll
                     for (int j = 0; j < 32; j += 8) {
                         if (col0 + j < p.N) {
-                            if (p.c_a) {
-                                float ca[8], cb[8];
-                                unpack8(__ldg(reinterpret_cast<const uint4*>(p.c_a + row_off + col0 + j)), ca);
-                                unpack8(__ldg(reinterpret_cast<const uint4*>(p.c_b + row_off + col0 + j)), cb);
-#pragma unroll
-                                for (int i = 0; i < 8; ++i) r[j + i] = __float_as_uint(__fmaf_rn(ca[i], __uint_as_float(r[j + i]), cb[i]));
-                            }
                             if (p.expert_ids) {
 #pragma unroll
                                 for (int i = 0; i < 8; ++i) r[j + i] = __float_as_uint(__uint_as_float(r[j + i]) * row_scale);
@@ -561,6 +600,11 @@ gemm_mxfp4_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             const bool row_ok = row < p.M;
             const int64_t row_off = ((int64_t)b * p.M + (row_ok ? row : 0)) * p.N;
             __nv_bfloat16* crow = p.C + row_off;
+            MulAddChunk ma;
+            if (p.c_a) {
+                prefetch_mul_add<BN>(p, row_off, nb * BN, row_ok);
+                ma.fetch(p, row_off, nb * BN, row_ok);
+            }
             if (!__all_sync(0xFFFFFFFFu, mbar_wait(tfull_bar(acc), acc_ph, abort_flag, p.status, kErrWaitEpilogue))) break;
             tc_fence_after();
             const uint32_t t_addr = tmem_base + lane_addr + acc * BN;
@@ -569,18 +613,15 @@ gemm_mxfp4_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                 uint32_t r[32];
                 tmem_ld32(t_addr + c, r);
                 tmem_ld_wait();
+                if (p.c_a) {
+                    ma.apply(r);
+                    if (c + 32 < BN) ma.fetch(p, row_off, nb * BN + c + 32, row_ok);
+                }
                 if (row_ok) {
                     const int col0 = nb * BN + c;
 #pragma unroll
                     for (int j = 0; j < 32; j += 8) {
                         if (col0 + j < p.N) {
-                            if (p.c_a) {
-                                float ca[8], cb[8];
-                                unpack8(__ldg(reinterpret_cast<const uint4*>(p.c_a + row_off + col0 + j)), ca);
-                                unpack8(__ldg(reinterpret_cast<const uint4*>(p.c_b + row_off + col0 + j)), cb);
-#pragma unroll
-                                for (int i = 0; i < 8; ++i) r[j + i] = __float_as_uint(__fmaf_rn(ca[i], __uint_as_float(r[j + i]), cb[i]));
-                            }
                             uint4 o;
                             __nv_bfloat162 q0 = __floats2bfloat162_rn(__uint_as_float(r[j + 0]), __uint_as_float(r[j + 1]));
                             __nv_bfloat162 q1 = __floats2bfloat162_rn(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
@@ -638,6 +679,20 @@ int launch_prepass(const SfJob& ja, const SfJob& jb, const GatherJob& jg, cudaSt
     return check_launch("mxfp4_prepass_kernel");
 }
 
+// 128 or 192 columns per tile of the one-CTA kernels.  A wave of tiles takes time in proportion to what the tensor core
+// reads from shared memory per K step (128 rows of A + bn rows of B) where the tiles share operands through L2, and to the
+// weight columns alone where every tile streams its own weights from HBM (`streams`: grouped calls with about one M
+// tile per expert); the width whose waves sum up to less wins.
+// M = 1000, N = 3080, K = 4224 with c_a / c_b: 19.0 us with 192 columns (136 tiles, one wave), 21.4 with 128 (200 tiles);
+// 8 experts of 8192 x 8192 with 16 rows each: 51.8 us with 128 columns (3.46 waves), 53.7 with 192 (2.32).
+int mxfp4_tile_width(int64_t m_blks, int64_t N, int64_t batch, int sms, bool streams) {
+    auto cost = [&](int bn) {
+        const int64_t tiles = m_blks * ((N + bn - 1) / bn) * batch;
+        return (tiles + sms - 1) / sms * (bn + (streams ? 0 : BM));
+    };
+    return cost(192) <= cost(128) ? 192 : 128;
+}
+
 // sfa_tc / sfb_tc: the scale pointer already is in the tensor-core layout (hkb_mxfp4_sf_to_tc or
 // hkb_quant_mxfp4_tc); otherwise it is row-major [batch, rows, K/32] and is re-laid-out into
 // per-(device, stream) scratch first.
@@ -659,11 +714,9 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
     Mxfp4Params p{};
     p.M = (int)M; p.N = (int)N; p.K = (int)K; p.batch = (int)batch;
     p.m_blks = (int)((M + BM - 1) / BM);
-    // wide tiles when there are enough of them to fill the SMs twice over
     const int sms = sm_count();
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
-    const bool wide = (int64_t)p.m_blks * ((N + 191) / 192) * batch >= 2LL * sms;
-    const int bn = wide ? 192 : 128;
+    const int bn = mxfp4_tile_width(p.m_blks, N, batch, sms, false);
     p.n_blks = (int)((N + bn - 1) / bn);
     p.sfa_rblks = sf_tc_rblks(M);
     p.sfb_rblks = sf_tc_rblks(N);
@@ -682,10 +735,10 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
     int rc = status_word(&p.status);
     if (rc != HKB_OK) return rc;
 
-    // CTA pairs on 256 x 192 tiles when there is at least half a wave of them (HKB_MXFP4_PAIRS=0: never)
+    // CTA pairs on 256 x 192 tiles when there are two waves of one-CTA tiles (HKB_MXFP4_PAIRS=0: never)
     static const bool pairs_on = [] { const char* v = getenv("HKB_MXFP4_PAIRS"); return !(v && v[0] == '0'); }();
     const int64_t pair_tiles = ((M + 255) / 256) * ((N + 191) / 192) * batch;
-    const bool pair = pairs_on && wide && M > 128 && pair_tiles >= sms / 2 && sms >= 2 && !sc;     // the split-cat store lives in the one-CTA kernels
+    const bool pair = pairs_on && (int64_t)p.m_blks * ((N + 191) / 192) * batch >= 2LL * sms && M > 128 && pair_tiles >= sms / 2 && sms >= 2 && !sc;     // the split-cat store lives in the one-CTA kernels
 
     const size_t sfa_bytes = (size_t)batch * p.sfa_rblks * p.katoms * 512;
     const size_t sfb_bytes = (size_t)batch * p.sfb_rblks * p.katoms * 512;
@@ -751,7 +804,7 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
     if (rc != HKB_OK) return rc;
     const int tiles = p.m_blks * p.n_blks * p.batch;
     const int grid = tiles < sms ? tiles : sms;
-    if (wide) {
+    if (bn == 192) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_mxfp4_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<192>::kDynamic);
         HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
         gemm_mxfp4_kernel<192><<<grid, 192, Cfg<192>::kDynamic, st>>>(tmA, tmB, p);
@@ -793,8 +846,7 @@ extern "C" int hkb_moe_gemm_mxfp4(const void* A, const void* B, void* C, const v
     p.m_blks = (int)(num_padded / BM);
     const int sms = sm_count();
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
-    const bool wide = (int64_t)p.m_blks * ((N + 191) / 192) >= 2LL * sms;
-    const int bn = wide ? 192 : 128;
+    const int bn = mxfp4_tile_width(p.m_blks, N, 1, sms, p.m_blks <= E);
     p.n_blks = (int)((N + bn - 1) / bn);
     p.sfa_rblks = sf_tc_rblks(num_padded);
     p.sfb_rblks = sf_tc_rblks(N);
@@ -830,7 +882,7 @@ extern "C" int hkb_moe_gemm_mxfp4(const void* A, const void* B, void* C, const v
     if (rc != HKB_OK) return rc;
     const int tiles = p.m_blks * p.n_blks;
     const int grid = tiles < sms ? tiles : sms;
-    if (wide) {
+    if (bn == 192) {
         HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<192>::kDynamic));
         gemm_mxfp4_kernel<192><<<grid, 192, Cfg<192>::kDynamic, st>>>(tmA, tmB, p);
         note_kernel("gemm_mxfp4_kernel<192> (grouped)");

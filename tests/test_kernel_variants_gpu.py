@@ -2,7 +2,8 @@
 import pytest
 import torch
 
-from test_gemm_gpu import DEV
+from oracle import gemm
+from test_gemm_gpu import DEV, _check, _dev, _mxfp4_operands, _status_ok
 
 pytestmark = pytest.mark.gpu
 
@@ -23,3 +24,19 @@ def test_mxfp4_scale_prepass_layout(hk, batch, rows, K):
     out = torch.full((mod.sf_tc_bytes(batch, rows, K),), 0xEE, dtype=torch.uint8, device=DEV)
     mod.sf_to_tc(sf if batch == 1 else sf.view(batch, rows, K // 32), out, K)
     assert torch.equal(out, _tc_layout(sf, batch, rows, K))
+
+
+@pytest.mark.parametrize("shape,kernel", [((1000, 3080, 384), "gemm_mxfp4_kernel<192>"), ((130, 136, 256), "gemm_mxfp4_kernel<128>"),
+                                          ((1100, 1904, 128), "gemm_mxfp4_kernel<128>")])
+def test_mxfp4_mul_add_and_tile_width_rule(hk, shape, kernel):
+    """Ragged rows and columns in the multiply-add epilogue of both tile widths, at sizes on either side of the width rule."""
+    M, N, K = shape
+    ac, wc, asc, wsc = _mxfp4_operands(M, N, K)
+    g = torch.Generator().manual_seed(3)
+    c_a, c_b = torch.randn(M, N, generator=g).bfloat16(), torch.randn(M, N, generator=g).bfloat16()
+    C = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    hk.fused_gemm.afp4wfp4_mul_add.dispatch(_dev(ac), _dev(wc), C, _dev(asc), _dev(wsc), _dev(c_a), _dev(c_b))
+    torch.cuda.synchronize()
+    assert hk.last_kernel() == kernel
+    _status_ok()
+    _check(C, gemm.mul_add(gemm.gemm_mxfp4(ac, wc, asc, wsc), c_a, c_b), f"mxfp4 mul_add {shape}")

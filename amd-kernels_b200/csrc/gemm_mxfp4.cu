@@ -735,6 +735,17 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
     int rc = status_word(&p.status);
     if (rc != HKB_OK) return rc;
 
+    // Decode shapes: HBM-bound on the weight stream; a kernel that deals the columns out evenly over the SMs and reads
+    // the scales in whichever layout they come (gemm_mxfp4_skinny.cu).  Microseconds, that kernel / the one below (with
+    // its pre-pass when row-major): 64 x 28672 x 8192 24.0 / 27.3, row-major 27.3 / 32.8; 16 x 14336 x 4096 10.7 / 13.2;
+    // 1 x 8192 x 2048 8.0 / 8.1; row-major 64 x 4096 x 4096 10.3 / 11.9.  Below two units per SM the tiles get too narrow
+    // to win without a pre-pass to save: 64 x 4096 x 4096 9.6 / 9.1, 16 x 1024 x 8192 13.1 / 11.7 with tensor-core scales.
+    const bool skinny_wins = N >= 32LL * sms || !(sfa_tc && sfb_tc);
+    if (M <= 64 && batch == 1 && N % 16 == 0 && aligned32(C) && !sc && skinny_wins) {
+        note_kernel("gemm_mxfp4_skinny_kernel");
+        return launch_gemm_mxfp4_skinny(A, B, C, sfa, sfb, sfa_tc, sfb_tc, c_a, c_b, M, N, K, p.status, st);
+    }
+
     // CTA pairs on 256 x 192 tiles when there are two waves of one-CTA tiles (HKB_MXFP4_PAIRS=0: never)
     static const bool pairs_on = [] { const char* v = getenv("HKB_MXFP4_PAIRS"); return !(v && v[0] == '0'); }();
     const int64_t pair_tiles = ((M + 255) / 256) * ((N + 191) / 192) * batch;

@@ -40,3 +40,30 @@ def test_mxfp4_mul_add_and_tile_width_rule(hk, shape, kernel):
     assert hk.last_kernel() == kernel
     _status_ok()
     _check(C, gemm.mul_add(gemm.gemm_mxfp4(ac, wc, asc, wsc), c_a, c_b), f"mxfp4 mul_add {shape}")
+
+
+@pytest.mark.parametrize("shape", [(1, 16, 128), (7, 2000, 384), (16, 10064, 256), (33, 17600, 128), (64, 9488, 1152), (64, 36000, 256)])
+def test_mxfp4_skinny_kernel(hk, shape):
+    """Tile widths of 1 to 15 units, one and two rounds, an odd number of K atoms, both layouts of either scale array."""
+    M, N, K = shape
+    ac, wc, asc, wsc = _mxfp4_operands(M, N, K)
+    ref = gemm.gemm_mxfp4(ac, wc, asc, wsc)
+    mod = hk.gemm.afp4wfp4
+    a, w, sa, sw = (_dev(v) for v in (ac, wc, asc, wsc))
+    a_tc = torch.full((mod.sf_tc_bytes(1, M, K),), 0xFF, dtype=torch.uint8, device=DEV)
+    w_tc = torch.full((mod.sf_tc_bytes(1, N, K),), 0xFF, dtype=torch.uint8, device=DEV)
+    mod.sf_to_tc(sa, a_tc, K)
+    mod.sf_to_tc(sw, w_tc, K)
+    for a_is_tc, b_is_tc in [(False, False), (True, True), (False, True), (True, False)]:
+        C = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        mod.dispatch_tc(a, w, C, a_tc if a_is_tc else sa, w_tc if b_is_tc else sw, a_is_tc, b_is_tc)
+        torch.cuda.synchronize()
+        wins = N >= 32 * torch.cuda.get_device_properties(0).multi_processor_count or not (a_is_tc and b_is_tc)
+        assert hk.last_kernel() == ("gemm_mxfp4_skinny_kernel" if wins else "gemm_mxfp4_kernel<128>")
+        _status_ok()
+        _check(C, ref, f"mxfp4 skinny {shape} {a_is_tc} {b_is_tc}")
+    g = torch.Generator().manual_seed(3)
+    c_a, c_b = torch.randn(M, N, generator=g).bfloat16(), torch.randn(M, N, generator=g).bfloat16()
+    hk.fused_gemm.afp4wfp4_mul_add.dispatch(a, w, C, sa, sw, _dev(c_a), _dev(c_b))
+    torch.cuda.synchronize()
+    _check(C, gemm.mul_add(ref, c_a, c_b), f"mxfp4 skinny mul_add {shape}")

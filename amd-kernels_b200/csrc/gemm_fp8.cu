@@ -1091,6 +1091,12 @@ int gemm_fp8_blockscale_impl(const void* A, const void* B, void* C, const float*
     p.wait_ns = kWaitLimitNs; p.skip_kblock = -1;
     rc = status_word(&p.status);
     if (rc != HKB_OK) return rc;
+    // Decode shapes: the weight stream bounds them (gemm_fp8_blockscale_skinny.cu).  At 32 tokens it is
+    // ahead for every N and K tried, at 64 behind (figures there).
+    if (M <= 32 && gn == 128 && !sc && n_peer == 0 && !trace) {
+        note_kernel("gemm_fp8_blockscale_skinny_kernel");
+        return launch_gemm_fp8_blockscale_skinny(A, B, C, sa, sb, c_a, c_b, M, N, K, ldc, p.status, (cudaStream_t)stream);
+    }
     p.m_blks = (int)((M + BM - 1) / BM);
     p.a_box_rows = BM;
     const int sms = sm_count();

@@ -23,6 +23,10 @@ int make_tmap_linear1k(CUtensorMap* map, const void* base, uint64_t bytes);
 int launch_gemm_fp8_skinny(const void* A, const void* B, void* C, const float* sa, const float* sb, const void* bias,
                            int64_t M, int64_t N, int64_t K, uint32_t* status, cudaStream_t st);
 
+// Block-scale FP8 GEMM for M <= 32, 128-column weight-scale groups (gemm_fp8_blockscale_skinny.cu); c_a / c_b or null.
+int launch_gemm_fp8_blockscale_skinny(const void* A, const void* B, void* C, const float* sa, const float* sb, const void* c_a, const void* c_b,
+                                      int64_t M, int64_t N, int64_t K, int64_t ldc, uint32_t* status, cudaStream_t st);
+
 // MXFP4 GEMM for M <= 64, batch 1, N % 16 == 0, C 32-byte aligned (gemm_mxfp4_skinny.cu); scales in either layout.
 int launch_gemm_mxfp4_skinny(const void* A, const void* B, void* C, const void* sfa, const void* sfb, bool sfa_tc, bool sfb_tc,
                              const void* c_a, const void* c_b, int64_t M, int64_t N, int64_t K, uint32_t* status, cudaStream_t st);

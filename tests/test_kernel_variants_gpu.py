@@ -67,3 +67,30 @@ def test_mxfp4_skinny_kernel(hk, shape):
     hk.fused_gemm.afp4wfp4_mul_add.dispatch(a, w, C, sa, sw, _dev(c_a), _dev(c_b))
     torch.cuda.synchronize()
     _check(C, gemm.mul_add(ref, c_a, c_b), f"mxfp4 skinny mul_add {shape}")
+
+
+@pytest.mark.parametrize("shape", [(1, 128, 128), (16, 2560, 640), (17, 14336, 1152), (32, 19072, 256), (8, 4096, 2048), (32, 40960, 128)])
+def test_blockscale_skinny_kernel(hk, shape):
+    """Tile heights of 1 to 8 units, one to three rounds, tiles across two scale groups, partial scale chunks and an odd number
+    of K blocks, both token widths; also bit-equal to the large kernel (whose result for rows 0..M of a taller A is the same sum in the same order)."""
+    M, N, K = shape
+    g = torch.Generator().manual_seed(M)
+    A = torch.randint(0, 255, (128, K), generator=g, dtype=torch.uint8)
+    B = torch.randint(0, 255, (N, K), generator=g, dtype=torch.uint8)
+    for t in (A, B):
+        t[(t & 0x7F) > 0x6F] = 0x38                                  # no NaN, magnitudes up to 120
+    sa = torch.rand(128, K // 128, generator=g) * 0.1 + 0.01
+    sb = torch.rand(K // 128, N // 128, generator=g) * 0.1 + 0.01
+    c_a, c_b = torch.randn(128, N, generator=g).bfloat16(), torch.randn(128, N, generator=g).bfloat16()
+    a, b, sad, sbd, ca, cb = (t.to(DEV) for t in (A, B, sa, sb, c_a, c_b))
+    big, big_ma = (torch.empty(128, N, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    C, C_ma = (torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    hk.gemm.a8w8_blockscale.dispatch(a, b, big, sad, sbd)
+    hk.fused_gemm.a8w8_blockscale_mul_add.dispatch(a, b, big_ma, sad, sbd, ca, cb)
+    hk.gemm.a8w8_blockscale.dispatch(a[:M], b, C, sad[:M], sbd)
+    assert hk.last_kernel() == "gemm_fp8_blockscale_skinny_kernel"
+    hk.fused_gemm.a8w8_blockscale_mul_add.dispatch(a[:M], b, C_ma, sad[:M], sbd, ca[:M], cb[:M])
+    torch.cuda.synchronize()
+    _status_ok()
+    _check(C, gemm.gemm_fp8_blockscale(A[:M].numpy(), B.numpy(), sa[:M], sb), f"blockscale skinny {shape}")
+    assert torch.equal(C, big[:M]) and torch.equal(C_ma, big_ma[:M])

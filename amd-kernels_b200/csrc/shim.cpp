@@ -34,11 +34,101 @@ struct TView {
 
 [[noreturn]] void fail(const std::string& m) { throw std::runtime_error(m); }
 
+// What a call needs from torch, looked up once: a pass of two calls spent about 30 us on the host, most of it in
+// attribute names built as strings, dtype reprs, a Python context manager and a Stream object per call.  Plain tensors (exactly
+// torch.Tensor or Parameter) are read through interned names and torch._C's own functions instead; everything else --
+// subclasses, duck-typed objects -- keeps the general path below.  Held for the life of the process, under the GIL.
+// 128 x 1024 x 1024, quantizer + GEMM: 29.7 us a pass before, 13.6 now; row-major MXFP4 with multiply-add 35.7 / 28.7.
+struct Torch {
+    PyObject *data_ptr, *shape, *dtype, *is_contiguous, *is_cuda, *get_device;      // interned attribute names
+    PyObject *tensor, *parameter;                                                   // types
+    PyObject *current_raw_stream, *exchange_device, *maybe_exchange_device;         // torch._C functions, all three or none
+    struct { PyObject* obj; std::string name; } dtypes[16];                         // torch.dtype objects are singletons
+    int n_dtypes = 0;
+};
+
+// Null while torch is not imported (then no argument can be one of its tensors).
+Torch* torch_cached() {
+    static Torch* T = nullptr;
+    if (T) return T;
+    py::object key = py::str("torch");
+    py::object mod = py::reinterpret_steal<py::object>(PyImport_GetModule(key.ptr()));
+    if (!mod) {
+        PyErr_Clear();
+        return nullptr;
+    }
+    if (!py::hasattr(mod, "nn") || !py::hasattr(mod, "Tensor")) return nullptr;      // still being imported
+    Torch* n = new Torch{};
+    n->data_ptr = PyUnicode_InternFromString("data_ptr");
+    n->shape = PyUnicode_InternFromString("shape");
+    n->dtype = PyUnicode_InternFromString("dtype");
+    n->is_contiguous = PyUnicode_InternFromString("is_contiguous");
+    n->is_cuda = PyUnicode_InternFromString("is_cuda");
+    n->get_device = PyUnicode_InternFromString("get_device");
+    n->tensor = py::object(mod.attr("Tensor")).release().ptr();
+    n->parameter = py::object(mod.attr("nn").attr("Parameter")).release().ptr();
+    py::object c = mod.attr("_C");
+    const char* const fns[3] = {"_cuda_getCurrentRawStream", "_cuda_exchangeDevice", "_cuda_maybeExchangeDevice"};
+    if (py::hasattr(c, fns[0]) && py::hasattr(c, fns[1]) && py::hasattr(c, fns[2])) {
+        n->current_raw_stream = py::object(c.attr(fns[0])).release().ptr();
+        n->exchange_device = py::object(c.attr(fns[1])).release().ptr();
+        n->maybe_exchange_device = py::object(c.attr(fns[2])).release().ptr();
+    }
+    return T = n;
+}
+
+py::object owned(PyObject* o) {
+    if (!o) throw py::error_already_set();
+    return py::reinterpret_steal<py::object>(o);
+}
+
+std::string dtype_name(const py::object& dtype) {
+    std::string s = py::str(dtype).cast<std::string>();
+    auto dot = s.rfind('.');
+    return dot == std::string::npos ? s : s.substr(dot + 1);
+}
+
+// view() below for a plain tensor: the same reads in the same order.
+TView view_tensor(Torch& T, PyObject* t, const char* name, bool need_contiguous) {
+    TView v;
+    v.none = false;
+    v.ptr = reinterpret_cast<void*>(owned(PyObject_CallMethodNoArgs(t, T.data_ptr)).cast<uint64_t>());
+    py::object shape = owned(PyObject_GetAttr(t, T.shape));
+    const Py_ssize_t rank = PyTuple_Size(shape.ptr());
+    if (rank < 0) throw py::error_already_set();
+    v.shape.resize((size_t)rank);
+    for (Py_ssize_t i = 0; i < rank; ++i) {
+        v.shape[i] = py::reinterpret_borrow<py::object>(PyTuple_GET_ITEM(shape.ptr(), i)).cast<int64_t>();
+        v.numel *= v.shape[i];
+    }
+    py::object dtype = owned(PyObject_GetAttr(t, T.dtype));
+    int d = 0;
+    while (d < T.n_dtypes && T.dtypes[d].obj != dtype.ptr()) ++d;
+    if (d < T.n_dtypes) {
+        v.dtype = T.dtypes[d].name;
+    } else {
+        v.dtype = dtype_name(dtype);
+        if (T.n_dtypes < (int)(sizeof T.dtypes / sizeof T.dtypes[0])) {
+            T.dtypes[T.n_dtypes].name = v.dtype;
+            T.dtypes[T.n_dtypes++].obj = dtype.release().ptr();
+        }
+    }
+    if (need_contiguous && owned(PyObject_CallMethodNoArgs(t, T.is_contiguous)).ptr() != Py_True)
+        fail(std::string(name) + ": tensor must be contiguous (row-major, inner stride 1)");
+    v.name = name;
+    if (owned(PyObject_GetAttr(t, T.is_cuda)).ptr() == Py_True) v.device = owned(PyObject_CallMethodNoArgs(t, T.get_device)).cast<int>();
+    return v;
+}
+
 TView view(const py::object& t, const char* name, bool allow_none = false, bool need_contiguous = true) {
     TView v;
     if (t.is_none()) {
         if (!allow_none) fail(std::string(name) + ": tensor is None");
         return v;
+    }
+    if (Torch* T = torch_cached()) {
+        PyObject* const type = reinterpret_cast<PyObject*>(Py_TYPE(t.ptr()));
+        if (type == T->tensor || type == T->parameter) return view_tensor(*T, t.ptr(), name, need_contiguous);
     }
     v.none = false;
     v.ptr = reinterpret_cast<void*>(t.attr("data_ptr")().cast<uint64_t>());
@@ -46,11 +136,7 @@ TView view(const py::object& t, const char* name, bool allow_none = false, bool 
         v.shape.push_back(d.cast<int64_t>());
         v.numel *= v.shape.back();
     }
-    if (py::hasattr(t, "dtype")) {
-        v.dtype = py::str(t.attr("dtype")).cast<std::string>();
-        auto dot = v.dtype.rfind('.');
-        if (dot != std::string::npos) v.dtype = v.dtype.substr(dot + 1);
-    }
+    if (py::hasattr(t, "dtype")) v.dtype = dtype_name(t.attr("dtype"));
     if (need_contiguous && py::hasattr(t, "is_contiguous") && !t.attr("is_contiguous")().cast<bool>())
         fail(std::string(name) + ": tensor must be contiguous (row-major, inner stride 1)");
     v.name = name;
@@ -89,18 +175,40 @@ void same_device(std::initializer_list<const TView*> vs) {
 // RAII: make the tensors' device current (through torch, which owns the CUDA context) and
 // fetch torch's current stream on it.
 struct Launch {
-    py::object guard;
+    py::object guard, previous;
     void* stream = nullptr;
     explicit Launch(int device) {
         if (device < 0) return;
+        Torch* const T = torch_cached();
+        if (T && T->current_raw_stream) {            // what the context manager and current_stream() below come to
+            py::object idx = py::int_(device);
+            previous = owned(PyObject_CallOneArg(T->exchange_device, idx.ptr()));
+            PyObject* const s = PyObject_CallOneArg(T->current_raw_stream, idx.ptr());
+            if (!s) {
+                py::error_already_set e;             // takes the error before the device is put back
+                restore();
+                throw e;
+            }
+            stream = reinterpret_cast<void*>(owned(s).cast<uint64_t>());
+            return;
+        }
         py::object cuda = py::module_::import("torch").attr("cuda");
         guard = cuda.attr("device")(device);
         guard.attr("__enter__")();
         stream = reinterpret_cast<void*>(cuda.attr("current_stream")(device).attr("cuda_stream").cast<uint64_t>());
     }
+    void restore() {
+        if (!previous) return;
+        PyObject* const r = PyObject_CallOneArg(torch_cached()->maybe_exchange_device, previous.ptr());
+        if (r) Py_DECREF(r); else PyErr_WriteUnraisable(nullptr);
+        previous = py::object();
+    }
     ~Launch() {
+        restore();
         if (guard) guard.attr("__exit__")(py::none(), py::none(), py::none());
     }
+    Launch(const Launch&) = delete;
+    Launch& operator=(const Launch&) = delete;
 };
 
 void check(int rc) {

@@ -94,3 +94,31 @@ def test_blockscale_skinny_kernel(hk, shape):
     _status_ok()
     _check(C, gemm.gemm_fp8_blockscale(A[:M].numpy(), B.numpy(), sa[:M], sb), f"blockscale skinny {shape}")
     assert torch.equal(C, big[:M]) and torch.equal(C_ma, big_ma[:M])
+
+
+def test_shim_reads_tensors_parameters_and_subclasses_alike(hk):
+    """Plain tensors and Parameters go through the native reads, subclasses through the general ones: same results, same
+    refusals, on the current stream of the tensors' device."""
+    class Sub(torch.Tensor):
+        pass
+
+    x = torch.randn(40, 256, generator=torch.Generator().manual_seed(1)).bfloat16().to(DEV)
+    want, ws = torch.empty(40, 256, dtype=torch.uint8, device=DEV), torch.empty(40, 1, device=DEV)
+    hk.per_token_quant_fwd(x, want, ws)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for wrap in (lambda t: t, lambda t: torch.nn.Parameter(t, requires_grad=False), lambda t: t.as_subclass(Sub)):
+        q, s = torch.zeros_like(want), torch.zeros_like(ws)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(1000000)                # a launch on another stream would overtake this and the zeros below
+            q.zero_()
+            hk.per_token_quant_fwd(wrap(x), wrap(q), wrap(s))
+        side.synchronize()
+        assert torch.equal(q, want) and torch.equal(s, ws)
+        with pytest.raises(RuntimeError, match="contiguous"):
+            hk.per_token_quant_fwd(wrap(x.T), wrap(q), wrap(s))
+        with pytest.raises(RuntimeError, match="dtype"):
+            hk.per_token_quant_fwd(wrap(x.half()), wrap(q), wrap(s))
+        with pytest.raises(RuntimeError, match="CUDA"):
+            hk.per_token_quant_fwd(wrap(x.cpu()), wrap(q), wrap(s))

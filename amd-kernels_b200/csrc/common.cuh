@@ -6,6 +6,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <utility>
 
 #include "../../include/hkb200.h"
 
@@ -32,6 +33,32 @@ inline int check_launch(const char* what) {
     if (e != cudaSuccess)
         return set_error(HKB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
     return HKB_OK;
+}
+
+// Launch whose grid may start before the kernel ahead of it in the stream has ended (programmatic dependent launch): its
+// blocks set up barriers, tensor memory and descriptors meanwhile.  EVERY thread of such a kernel calls pdl_wait() before
+// its first access to global memory -- operands, results, scratch -- so that all earlier work has completed and is visible;
+// that also keeps the chain whole when the next kernel is launched this way in turn.  cluster: CTAs per cluster, 0 = none.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, unsigned cluster, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cluster) {
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = cluster;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
+    }
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -61,6 +88,10 @@ uint32_t* static_status_peek();
 
 // ---- device helpers -----------------------------------------------------------------------
 namespace hkb {
+
+// See launch_dependent().  pdl_trigger: the kernel behind this one may be launched once every block has come this far.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }

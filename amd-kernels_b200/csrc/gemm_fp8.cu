@@ -309,6 +309,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if constexpr (kPair) tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
         else tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
     }
+    pdl_wait();      // nothing in global memory is touched before this
     tc_fence_before();
     __syncthreads();
     if constexpr (kPair) { __syncwarp(); cluster_sync_all(); }   // the partner's barriers and TMEM exist before anyone signals them
@@ -757,6 +758,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const uint8_t* __restrict__ x, const float* __restrict__ xs, const int32_t* __restrict__ gather, int n_act,
                        uint8_t* __restrict__ xg, float* __restrict__ xsg, int64_t rows, int K, int kblocks, int64_t tokens) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= rows) return;
     const int lane = threadIdx.x & 31;
@@ -804,19 +807,7 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmP
     const int tiles = p.m_blks * p.n_blks * p.batch;
     int clusters = sms / 2;
     if (tiles < clusters) clusters = tiles;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * clusters);
-    cfg.blockDim = dim3(gemm_threads<256, kBlockScale, true>());
-    cfg.dynamicSmemBytes = L::kDynamic;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p);
+    e = launch_dependent(kern, 2 * clusters, gemm_threads<256, kBlockScale, true>(), L::kDynamic, 2, st, tmA, tmB, p);
     HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cluster launch of gemm_fp8_kernel failed: %s", cudaGetErrorString(e));
     note_kernel(kBlockScale ? "gemm_fp8_kernel<256,blockscale,pair>" : "gemm_fp8_kernel<256,pts,pair>");
     return check_launch("gemm_fp8_kernel (CTA pairs)");
@@ -852,7 +843,7 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams
     const int sms = sm_count();
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
     const int grid = tiles < sms ? tiles : sms;
-    kern<<<grid, gemm_threads<BN, kBlockScale>(), L::kDynamic, st>>>(tmA, tmB, p);
+    HKB_CUDA(launch_dependent(kern, grid, gemm_threads<BN, kBlockScale>(), L::kDynamic, 0, st, tmA, tmB, p));
     note_kernel(kOut == 1 ? (BN == 256 ? "gemm_fp8_kernel<256,blockscale,scatter>" : "gemm_fp8_kernel<128,blockscale,scatter>") :
                 kOut == 2 ? (kGn128 ? "gemm_fp8_kernel<128,blockscale,split_cat>" : "gemm_fp8_kernel<128,blockscale,gn1,split_cat>") :
                 kOut == 3 ? (BN == 256 ? "gemm_fp8_kernel<256,blockscale,grouped>" : "gemm_fp8_kernel<128,blockscale,grouped>") :
@@ -1005,8 +996,8 @@ int hkb_moe_gemm_fp8_blockscale(const void* X, const void* W, void* Y, const flo
         if (rc != HKB_OK) return rc;
         rc = scratch_get(SCRATCH_SFB, st, (size_t)rows * kblocks * 4, &xsg);
         if (rc != HKB_OK) return rc;
-        moe_gather_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const uint8_t*)X, X_scale, GatherIndx, (int)n_expts_act,
-                                                                             (uint8_t*)xg, (float*)xsg, rows, (int)K, kblocks, tokens);
+        HKB_CUDA(launch_dependent(moe_gather_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, 0, st, (const uint8_t*)X, X_scale, GatherIndx,
+                                  (int)n_expts_act, (uint8_t*)xg, (float*)xsg, rows, (int)K, kblocks, tokens));
         rc = check_launch("moe_gather_rows_kernel");
         if (rc != HKB_OK) return rc;
         A = xg;

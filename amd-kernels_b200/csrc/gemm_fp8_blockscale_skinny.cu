@@ -111,6 +111,7 @@ gemm_fp8_blockscale_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+    pdl_wait();      // nothing in global memory is touched before this
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -311,7 +312,7 @@ template <int NT>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB0, const CUtensorMap& tmB1, const BsSkinnyParams& p, int smem, int grid, cudaStream_t st) {
     const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_blockscale_skinny_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", smem, cudaGetErrorString(e));
-    gemm_fp8_blockscale_skinny_kernel<NT><<<grid, kThreads, smem, st>>>(tmA, tmB0, tmB1, p);
+    HKB_CUDA(launch_dependent(gemm_fp8_blockscale_skinny_kernel<NT>, grid, kThreads, smem, 0, st, tmA, tmB0, tmB1, p));
     return check_launch("gemm_fp8_blockscale_skinny_kernel");
 }
 

@@ -93,6 +93,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), TMEM_COLS);
+    pdl_wait();      // nothing in global memory is touched before this
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -262,7 +263,7 @@ int launch_gemm_fp8_skinny(const void* A, const void* B, void* C, const float* s
     const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", smem, cudaGetErrorString(e));
     const int grid = p.tiles < sms ? p.tiles : sms;
-    gemm_fp8_skinny_kernel<<<grid, 192, smem, st>>>(tmA, tmB128, tmB64, tmB16, p);
+    HKB_CUDA(launch_dependent(gemm_fp8_skinny_kernel, grid, 192, smem, 0, st, tmA, tmB128, tmB64, tmB16, p));
     return check_launch("gemm_fp8_skinny_kernel");
 }
 

@@ -65,6 +65,7 @@ template <int NW, int TPR, bool INT8>
 __global__ void __launch_bounds__(256, NW <= 4 ? 4 : 2)
 quant_row_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
                  float* __restrict__ scales, int64_t M, int nwide, int64_t ldx) {
+    pdl_trigger();
     constexpr int RPB = 256 / TPR;
     const int tid = threadIdx.x;
     const int r_in = tid / TPR;
@@ -196,6 +197,7 @@ template <int ITER>
 __global__ void __launch_bounds__(256)
 quant_1x128_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
                    float* __restrict__ scales, int64_t total_groups) {
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane & 3;
     const int64_t g0 = ((int64_t)blockIdx.x * 8 + warp) * (8 * ITER) + (lane >> 2);
@@ -234,6 +236,7 @@ template <int NW, int TPR>
 __global__ void __launch_bounds__(256, NW <= 4 ? 3 : 2)
 rmsnorm_quant_1x128_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                            uint8_t* __restrict__ q, float* __restrict__ scales, int64_t M, int nwide, float eps) {
+    pdl_trigger();
     constexpr int RPB = 256 / TPR;
     const int tid = threadIdx.x;
     const int r_in = tid / TPR;

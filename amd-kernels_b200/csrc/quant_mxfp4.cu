@@ -103,6 +103,7 @@ template <int MODE, int ITER, bool TC = false>
 __global__ void __launch_bounds__(256)
 quant_mxfp4_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ codes,
                    uint8_t* __restrict__ scales, int64_t total_blocks, const SfTc tc = SfTc{}) {
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = lane & 1;
     const int64_t b0 = ((int64_t)blockIdx.x * 8 + warp) * (16 * ITER) + (lane >> 1);
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(256, NW <= 4 ? 3 : 2)
 rmsnorm_quant_mxfp4_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                            uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int64_t M, int nwide, float eps,
                            const SfTc tc) {
+    pdl_trigger();
     constexpr int RPB = 256 / TPR;
     const int tid = threadIdx.x;
     const int lane = tid & 31;

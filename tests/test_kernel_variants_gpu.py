@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from oracle import gemm
-from test_gemm_gpu import DEV, _check, _dev, _mxfp4_operands, _status_ok
+from test_gemm_gpu import DEV, _check, _dev, _fp8_operands, _mxfp4_operands, _status_ok
 
 pytestmark = pytest.mark.gpu
 
@@ -122,3 +122,21 @@ def test_shim_reads_tensors_parameters_and_subclasses_alike(hk):
             hk.per_token_quant_fwd(wrap(x.half()), wrap(q), wrap(s))
         with pytest.raises(RuntimeError, match="CUDA"):
             hk.per_token_quant_fwd(wrap(x.cpu()), wrap(q), wrap(s))
+
+
+@pytest.mark.parametrize("batch,M,N,K,with_bias", [(8, 512, 4096, 128, True), (1, 2300, 6408, 256, False), (2, 1290, 5000, 384, True)])
+def test_per_token_pairs_split_last_wave(hk, batch, M, N, K, with_bias):
+    """256 x 256 tiles whose last wave is mostly empty and walked as halves; rows, columns and halves past the edges."""
+    aq, bq, sa, sb = _fp8_operands(M, N, K, batch)
+    bias = torch.randn(batch, N, generator=torch.Generator().manual_seed(2)).bfloat16() if with_bias else None
+    C = torch.full((batch, M, N) if batch > 1 else (M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    if batch > 1:
+        hk.batched_gemm.a8w8.dispatch(_dev(aq), _dev(bq), _dev(sa), _dev(sb), C, None if bias is None else _dev(bias))
+    else:
+        hk.gemm.a8w8_per_token.dispatch(_dev(aq), _dev(bq), C, _dev(sa), _dev(sb))
+    torch.cuda.synchronize()
+    assert hk.last_kernel() == "gemm_fp8_kernel<256,pts,pair>"
+    tiles, clusters = batch * -(-M // 256) * -(-N // 256), torch.cuda.get_device_properties(0).multi_processor_count // 2
+    assert tiles > clusters and 0 < 2 * (tiles % clusters) <= clusters or clusters != 74
+    _status_ok()
+    _check(C, gemm.gemm_fp8_per_token(aq, bq, sa, sb, bias), f"per-token pairs {batch}x{M}x{N}x{K}")

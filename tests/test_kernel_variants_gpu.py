@@ -140,3 +140,45 @@ def test_per_token_pairs_split_last_wave(hk, batch, M, N, K, with_bias):
     assert tiles > clusters and 0 < 2 * (tiles % clusters) <= clusters or clusters != 74
     _status_ok()
     _check(C, gemm.gemm_fp8_per_token(aq, bq, sa, sb, bias), f"per-token pairs {batch}x{M}x{N}x{K}")
+
+
+@pytest.mark.parametrize("M", [16, 300])
+def test_dependent_launches_under_graph_capture(hk, M):
+    """Quantizer and GEMMs captured as one chain of programmatic launches: replays follow the inputs, kernel after kernel."""
+    N, K = 5120, 1024
+    g = torch.Generator().manual_seed(M)
+    w = (torch.randn(N, K, generator=g) * 0.02).bfloat16().to(DEV)
+    x = torch.zeros(M, K, dtype=torch.bfloat16, device=DEV)
+    mod = hk.gemm.afp4wfp4
+    u8 = lambda *s: torch.zeros(*s, dtype=torch.uint8, device=DEV)      # noqa: E731
+    f32 = lambda *s: torch.zeros(*s, device=DEV)                         # noqa: E731
+    wq, ws, xq, xs = u8(N, K), f32(N, 1), u8(M, K), f32(M, 1)
+    bq, bs, yq, ys = u8(N, K), f32(K // 128, N // 128), u8(M, K), f32(M, K // 128)
+    fq, fs, zq, zs = u8(N, K // 2), u8(mod.sf_tc_bytes(1, N, K)), u8(M, K // 2), u8(mod.sf_tc_bytes(1, M, K))
+    hk.per_token_quant_fwd(w, wq, ws)
+    hk.weight_quant_128x128(w, bq, bs)
+    hk.fused_rmsnorm_mxfp4_quant_tc_fwd(w, None, fq, None, fs, 1e-6)
+    C = [torch.zeros(M, N, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+
+    def chain():
+        hk.per_token_quant_fwd(x, xq, xs)
+        hk.gemm.a8w8_per_token.dispatch(xq, wq, C[0], xs, ws)
+        hk.fused_rmsnorm_fp8_quant_fwd(x, None, yq, ys, 1e-6)
+        hk.gemm.a8w8_blockscale.dispatch(yq, bq, C[1], ys, bs)
+        hk.fused_rmsnorm_mxfp4_quant_tc_fwd(x, None, zq, None, zs, 1e-6)
+        mod.dispatch_tc(zq, fq, C[2], zs, fs, True, True)
+
+    chain()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for seed in range(8):
+        x.copy_(torch.randn(M, K, generator=torch.Generator().manual_seed(seed)).bfloat16())
+        chain()
+        want = [c.clone() for c in C]
+        for c in C:
+            c.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(c, v) for c, v in zip(C, want)) and want[0].abs().max() > 0
+    _status_ok()

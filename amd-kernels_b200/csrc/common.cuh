@@ -39,27 +39,35 @@ inline int check_launch(const char* what) {
 // blocks set up barriers, tensor memory and descriptors meanwhile.  EVERY thread of such a kernel calls pdl_wait() before
 // its first access to global memory -- operands, results, scratch -- so that all earlier work has completed and is visible;
 // that also keeps the chain whole when the next kernel is launched this way in turn.  cluster: CTAs per cluster, 0 = none.
+// early = false: an ordinary launch of the same kernel.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, unsigned cluster, cudaStream_t st, Args&&... args) {
+cudaError_t launch_dependent(bool early, void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, unsigned cluster, cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 0;
+    if (early) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
     if (cluster) {
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = cluster;
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.numAttrs = 2;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
     }
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
+
+// Whether a persistent GEMM starts early.  Blocks that start early land on the SMs in the order in which the quantizer
+// leaves them, which costs the long kernels some of the L2 sharing between neighbouring tiles, and a launch latency is
+// nothing to them: 16384 x 57344 x 8192 block-scale took 8.71 ms a pass early and 8.54 not, 4096 x 14336 x 4096 (12 tiles per
+// block) 310 us against 305; at 3.5 tiles per pair (8 x 512 x 4096 x 4096 per-token) 83.2 us early and 84.1 not.
+inline bool starts_early(int64_t tiles, int64_t workers) { return tiles <= 4 * workers; }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

@@ -825,7 +825,7 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     // 8 x 512 x 4096 x 4096 (256 tiles on 74 clusters, 3.46 waves): quantizer + GEMM 68.9 us a pass whole, 67.1 split.
     const int last = tiles % clusters;
     p.split_from = tiles > clusters && 2 * last <= clusters ? tiles - last : tiles;
-    e = launch_dependent(kern, 2 * clusters, gemm_threads<256, kBlockScale, true>(), L::kDynamic, 2, st, tmA, tmB, p, tmBHalf);
+    e = launch_dependent(starts_early(tiles, clusters), kern, 2 * clusters, gemm_threads<256, kBlockScale, true>(), L::kDynamic, 2, st, tmA, tmB, p, tmBHalf);
     HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cluster launch of gemm_fp8_kernel failed: %s", cudaGetErrorString(e));
     note_kernel(kBlockScale ? "gemm_fp8_kernel<256,blockscale,pair>" : "gemm_fp8_kernel<256,pts,pair>");
     return check_launch("gemm_fp8_kernel (CTA pairs)");
@@ -861,7 +861,7 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams
     const int sms = sm_count();
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
     const int grid = tiles < sms ? tiles : sms;
-    HKB_CUDA(launch_dependent(kern, grid, gemm_threads<BN, kBlockScale>(), L::kDynamic, 0, st, tmA, tmB, p, tmB));
+    HKB_CUDA(launch_dependent(starts_early(tiles, grid), kern, grid, gemm_threads<BN, kBlockScale>(), L::kDynamic, 0, st, tmA, tmB, p, tmB));
     note_kernel(kOut == 1 ? (BN == 256 ? "gemm_fp8_kernel<256,blockscale,scatter>" : "gemm_fp8_kernel<128,blockscale,scatter>") :
                 kOut == 2 ? (kGn128 ? "gemm_fp8_kernel<128,blockscale,split_cat>" : "gemm_fp8_kernel<128,blockscale,gn1,split_cat>") :
                 kOut == 3 ? (BN == 256 ? "gemm_fp8_kernel<256,blockscale,grouped>" : "gemm_fp8_kernel<128,blockscale,grouped>") :
@@ -1017,7 +1017,7 @@ int hkb_moe_gemm_fp8_blockscale(const void* X, const void* W, void* Y, const flo
         if (rc != HKB_OK) return rc;
         rc = scratch_get(SCRATCH_SFB, st, (size_t)rows * kblocks * 4, &xsg);
         if (rc != HKB_OK) return rc;
-        HKB_CUDA(launch_dependent(moe_gather_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, 0, st, (const uint8_t*)X, X_scale, GatherIndx,
+        HKB_CUDA(launch_dependent(true, moe_gather_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, 0, st, (const uint8_t*)X, X_scale, GatherIndx,
                                   (int)n_expts_act, (uint8_t*)xg, (float*)xsg, rows, (int)K, kblocks, tokens));
         rc = check_launch("moe_gather_rows_kernel");
         if (rc != HKB_OK) return rc;

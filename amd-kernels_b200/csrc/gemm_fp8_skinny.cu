@@ -265,7 +265,7 @@ int launch_gemm_fp8_skinny(const void* A, const void* B, void* C, const float* s
     const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", smem, cudaGetErrorString(e));
     const int grid = p.tiles < sms ? p.tiles : sms;
-    HKB_CUDA(launch_dependent(gemm_fp8_skinny_kernel, grid, 192, smem, 0, st, tmA, tmB0, tmB1, p));
+    HKB_CUDA(launch_dependent(true, gemm_fp8_skinny_kernel, grid, 192, smem, 0, st, tmA, tmB0, tmB1, p));
     return check_launch("gemm_fp8_skinny_kernel");
 }
 

@@ -679,7 +679,7 @@ int launch_prepass(const SfJob& ja, const SfJob& jb, const GatherJob& jg, cudaSt
     const int64_t blocks = (int64_t)ja.blocks + jb.blocks + jg.blocks;
     if (blocks == 0) return HKB_OK;
     HKB_REQUIRE(blocks < (1LL << 31), HKB_ERR_BAD_SHAPE, "mxfp4 scale layout: too many row blocks");
-    HKB_CUDA(launch_dependent(mxfp4_prepass_kernel, (unsigned)blocks, 256, 0, 0, st, ja, jb, jg));
+    HKB_CUDA(launch_dependent(true, mxfp4_prepass_kernel, (unsigned)blocks, 256, 0, 0, st, ja, jb, jg));
     return check_launch("mxfp4_prepass_kernel");
 }
 
@@ -798,7 +798,7 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
         HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
         int clusters = sms / 2;
         if (pair_tiles < clusters) clusters = (int)pair_tiles;
-        e = launch_dependent(gemm_mxfp4_pair_kernel, 2 * clusters, 192, PairCfg::kDynamic, 2, st, tmA, tmB, tmSfa, tmSfb, pp);
+        e = launch_dependent(starts_early(pair_tiles, clusters), gemm_mxfp4_pair_kernel, 2 * clusters, 192, PairCfg::kDynamic, 2, st, tmA, tmB, tmSfa, tmSfb, pp);
         HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "launch of gemm_mxfp4_pair_kernel failed: %s", cudaGetErrorString(e));
         note_kernel("gemm_mxfp4_pair_kernel<256x192>");
         return check_launch("gemm_mxfp4_pair_kernel");
@@ -810,12 +810,12 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
     if (bn == 192) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_mxfp4_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<192>::kDynamic);
         HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
-        HKB_CUDA(launch_dependent(gemm_mxfp4_kernel<192>, grid, 192, Cfg<192>::kDynamic, 0, st, tmA, tmB, p));
+        HKB_CUDA(launch_dependent(starts_early(tiles, sms), gemm_mxfp4_kernel<192>, grid, 192, Cfg<192>::kDynamic, 0, st, tmA, tmB, p));
         note_kernel("gemm_mxfp4_kernel<192>");
     } else {
         const cudaError_t e = cudaFuncSetAttribute(gemm_mxfp4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<128>::kDynamic);
         HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
-        HKB_CUDA(launch_dependent(gemm_mxfp4_kernel<128>, grid, 192, Cfg<128>::kDynamic, 0, st, tmA, tmB, p));
+        HKB_CUDA(launch_dependent(starts_early(tiles, sms), gemm_mxfp4_kernel<128>, grid, 192, Cfg<128>::kDynamic, 0, st, tmA, tmB, p));
         note_kernel("gemm_mxfp4_kernel<128>");
     }
     return check_launch("gemm_mxfp4_kernel");
@@ -887,11 +887,11 @@ extern "C" int hkb_moe_gemm_mxfp4(const void* A, const void* B, void* C, const v
     const int grid = tiles < sms ? tiles : sms;
     if (bn == 192) {
         HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<192>::kDynamic));
-        HKB_CUDA(launch_dependent(gemm_mxfp4_kernel<192>, grid, 192, Cfg<192>::kDynamic, 0, st, tmA, tmB, p));
+        HKB_CUDA(launch_dependent(starts_early(tiles, sms), gemm_mxfp4_kernel<192>, grid, 192, Cfg<192>::kDynamic, 0, st, tmA, tmB, p));
         note_kernel("gemm_mxfp4_kernel<192> (grouped)");
     } else {
         HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<128>::kDynamic));
-        HKB_CUDA(launch_dependent(gemm_mxfp4_kernel<128>, grid, 192, Cfg<128>::kDynamic, 0, st, tmA, tmB, p));
+        HKB_CUDA(launch_dependent(starts_early(tiles, sms), gemm_mxfp4_kernel<128>, grid, 192, Cfg<128>::kDynamic, 0, st, tmA, tmB, p));
         note_kernel("gemm_mxfp4_kernel<128> (grouped)");
     }
     return check_launch("gemm_mxfp4_kernel");
@@ -1063,7 +1063,7 @@ extern "C" int hkb_gemm_mxfp4_static(const void* A, const void* B, void* C, cons
     const int tiles = p.m_blks * p.n_blks * p.batch;
     const int sms = sm_count();
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
-    HKB_CUDA(launch_dependent(gemm_mxfp4_kernel<128>, tiles < sms ? tiles : sms, 192, Cfg<128>::kDynamic, 0, st, tmA, tmB, p));
+    HKB_CUDA(launch_dependent(starts_early(tiles, sms), gemm_mxfp4_kernel<128>, tiles < sms ? tiles : sms, 192, Cfg<128>::kDynamic, 0, st, tmA, tmB, p));
     note_kernel("gemm_mxfp4_kernel<128> (static scratch)");
     return check_launch("gemm_mxfp4_kernel");
 }

@@ -20,10 +20,18 @@ int set_error(int code, const char* fmt, ...);
         if (!(cond)) return ::hkb::set_error((code), __VA_ARGS__); \
     } while (0)
 
+// A failed runtime call also leaves its error pending for the thread, where the next launch check -- this library's or that of
+// anything else in the process that shares the runtime, torch for one -- would find it and report a launch that went well as
+// failed.  So whoever sees a failure takes it back here.
+inline bool cuda_ok(cudaError_t e) {
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+}
+
 #define HKB_CUDA(call)                                                              \
     do {                                                                            \
-        cudaError_t e__ = (call);                                                   \
-        if (e__ != cudaSuccess)                                                     \
+        const cudaError_t e__ = (call);                                             \
+        if (!::hkb::cuda_ok(e__))                                                   \
             return ::hkb::set_error(HKB_ERR_CUDA, "%s failed: %s", #call,           \
                                     cudaGetErrorString(e__));                       \
     } while (0)

@@ -39,7 +39,7 @@ void load_encoder() {
     std::call_once(g_encode_once, [] {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess &&
+        if (cuda_ok(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q)) &&
             q == cudaDriverEntryPointSuccess)
             g_encode = reinterpret_cast<EncodeFn>(fn);
     });
@@ -814,8 +814,7 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     using L = SmemLayout<256, STAGES, true, BM, kBlockScale ? 256 : 0>;
     static_assert(L::kDynamic <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
     auto kern = gemm_fp8_kernel<256, STAGES, kBlockScale, true, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
-    HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", L::kDynamic, cudaGetErrorString(e));
+    HKB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic));
     const int sms = sm_count();
     HKB_REQUIRE(sms > 1, HKB_ERR_CUDA, "no CUDA device");
     const int tiles = p.m_blks * p.n_blks * p.batch;
@@ -825,8 +824,8 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     // 8 x 512 x 4096 x 4096 (256 tiles on 74 clusters, 3.46 waves): quantizer + GEMM 68.9 us a pass whole, 67.1 split.
     const int last = tiles % clusters;
     p.split_from = tiles > clusters && 2 * last <= clusters ? tiles - last : tiles;
-    e = launch_dependent(starts_early(tiles, clusters), kern, 2 * clusters, gemm_threads<256, kBlockScale, true>(), L::kDynamic, 2, st, tmA, tmB, p, tmBHalf);
-    HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cluster launch of gemm_fp8_kernel failed: %s", cudaGetErrorString(e));
+    const int threads = gemm_threads<256, kBlockScale, true>();
+    HKB_CUDA(launch_dependent(starts_early(tiles, clusters), kern, 2 * clusters, threads, L::kDynamic, 2, st, tmA, tmB, p, tmBHalf));
     note_kernel(kBlockScale ? "gemm_fp8_kernel<256,blockscale,pair>" : "gemm_fp8_kernel<256,pts,pair>");
     return check_launch("gemm_fp8_kernel (CTA pairs)");
 }
@@ -855,8 +854,7 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams
     static_assert(L::kDynamic <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
     auto kern = gemm_fp8_kernel<BN, STAGES, kBlockScale, kGn128, false, AROWS, kOut>;
     // the attribute is per device; set it on every call (cheap) so multi-device processes work
-    const cudaError_t attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic);
-    HKB_REQUIRE(attr_err == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", L::kDynamic, cudaGetErrorString(attr_err));
+    HKB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic));
     const int tiles = p.m_blks * p.n_blks * p.batch;
     const int sms = sm_count();
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
@@ -980,8 +978,7 @@ int hkb_debug_gemm_fp8_blockscale_timeline(const void* A, const void* B, void* C
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
     const int64_t need = (int64_t)sms * kTraceEvents * kTraceKb * 8;
     HKB_REQUIRE(trace_bytes >= need, HKB_ERR_BAD_ARG, "gemm_fp8_blockscale timeline: trace buffer has %lld bytes, %lld needed", (long long)trace_bytes, (long long)need);
-    const cudaError_t e = cudaMemsetAsync(trace, 0, (size_t)need, (cudaStream_t)stream);
-    HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaMemsetAsync failed: %s", cudaGetErrorString(e));
+    HKB_CUDA(cudaMemsetAsync(trace, 0, (size_t)need, (cudaStream_t)stream));
     return gemm_fp8_blockscale_impl(A, B, C, sa, sb, 128, nullptr, nullptr, M, N, K, stream, 0, nullptr, 0, nullptr, (unsigned long long*)trace);
 }
 

@@ -310,8 +310,7 @@ gemm_fp8_blockscale_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const
 
 template <int NT>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB0, const CUtensorMap& tmB1, const BsSkinnyParams& p, int smem, int grid, cudaStream_t st) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_blockscale_skinny_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", smem, cudaGetErrorString(e));
+    HKB_CUDA(cudaFuncSetAttribute(gemm_fp8_blockscale_skinny_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     HKB_CUDA(launch_dependent(true, gemm_fp8_blockscale_skinny_kernel<NT>, grid, kThreads, smem, 0, st, tmA, tmB0, tmB1, p));
     return check_launch("gemm_fp8_blockscale_skinny_kernel");
 }

@@ -794,12 +794,10 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
         if (rc != HKB_OK) return rc;
         rc = make_tmap_linear1k(&tmSfb, sfb_sw, sfb_bytes);
         if (rc != HKB_OK) return rc;
-        cudaError_t e = cudaFuncSetAttribute(gemm_mxfp4_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::kDynamic);
-        HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
+        HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::kDynamic));
         int clusters = sms / 2;
         if (pair_tiles < clusters) clusters = (int)pair_tiles;
-        e = launch_dependent(starts_early(pair_tiles, clusters), gemm_mxfp4_pair_kernel, 2 * clusters, 192, PairCfg::kDynamic, 2, st, tmA, tmB, tmSfa, tmSfb, pp);
-        HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "launch of gemm_mxfp4_pair_kernel failed: %s", cudaGetErrorString(e));
+        HKB_CUDA(launch_dependent(starts_early(pair_tiles, clusters), gemm_mxfp4_pair_kernel, 2 * clusters, 192, PairCfg::kDynamic, 2, st, tmA, tmB, tmSfa, tmSfb, pp));
         note_kernel("gemm_mxfp4_pair_kernel<256x192>");
         return check_launch("gemm_mxfp4_pair_kernel");
     }
@@ -808,13 +806,11 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
     const int tiles = p.m_blks * p.n_blks * p.batch;
     const int grid = tiles < sms ? tiles : sms;
     if (bn == 192) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_mxfp4_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<192>::kDynamic);
-        HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
+        HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<192>::kDynamic));
         HKB_CUDA(launch_dependent(starts_early(tiles, sms), gemm_mxfp4_kernel<192>, grid, 192, Cfg<192>::kDynamic, 0, st, tmA, tmB, p));
         note_kernel("gemm_mxfp4_kernel<192>");
     } else {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_mxfp4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<128>::kDynamic);
-        HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
+        HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<128>::kDynamic));
         HKB_CUDA(launch_dependent(starts_early(tiles, sms), gemm_mxfp4_kernel<128>, grid, 192, Cfg<128>::kDynamic, 0, st, tmA, tmB, p));
         note_kernel("gemm_mxfp4_kernel<128>");
     }
@@ -1005,7 +1001,7 @@ int static_addresses(StaticSlot* out) {
 
 uint32_t* static_status_peek() {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    if (!cuda_ok(cudaGetDevice(&dev)) || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lk(g_static_mu);
     return g_static_slot[dev].status;
 }

@@ -320,8 +320,7 @@ int launch_gemm_mxfp4_skinny(const void* A, const void* B, void* C, const void* 
     if (rc != HKB_OK) return rc;
     rc = make_tmap_bytes(&tmB16, B, (uint64_t)K / 2, (uint64_t)N, 1, 16);
     if (rc != HKB_OK) return rc;
-    const cudaError_t e = cudaFuncSetAttribute(gemm_mxfp4_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    HKB_REQUIRE(e == cudaSuccess, HKB_ERR_CUDA, "cudaFuncSetAttribute(smem=%d) failed: %s", smem, cudaGetErrorString(e));
+    HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const int grid = p.tiles < sms ? p.tiles : sms;
     HKB_CUDA(launch_dependent(true, gemm_mxfp4_skinny_kernel, grid, 192 + 32 * kStagers, smem, 0, st, tmA, tmB128, tmB64, tmB16, p));
     return check_launch("gemm_mxfp4_skinny_kernel");

@@ -49,7 +49,7 @@ int sm_count() {
     std::lock_guard<std::mutex> lk(g_mu);
     if (g_dev[dev].sms == 0) {
         int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+        if (!cuda_ok(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev))) return 0;
         g_dev[dev].sms = n;
     }
     return g_dev[dev].sms;
@@ -139,10 +139,7 @@ int hkb_shard_bounds(int64_t N, int64_t world_size, int64_t rank, int64_t* n0, i
 int hkb_release(void) {
     using namespace hkb;
     int ndev = 0;
-    if (cudaGetDeviceCount(&ndev) != cudaSuccess) {
-        cudaGetLastError();
-        return HKB_OK;  // nothing can have been allocated without a device
-    }
+    if (!cuda_ok(cudaGetDeviceCount(&ndev))) return HKB_OK;  // nothing can have been allocated without a device
     int prev = 0;
     HKB_CUDA(cudaGetDevice(&prev));
     std::lock_guard<std::mutex> lk(g_mu);
@@ -185,7 +182,7 @@ int hkb_check_status(void* stream) {
     HKB_CUDA(cudaStreamSynchronize(st));
     if (host[0] | host[1]) {
         for (int i = 0; i < 2; ++i)
-            if (host[i]) cudaMemsetAsync(words[i], 0, sizeof(uint32_t), st);
+            if (host[i]) cuda_ok(cudaMemsetAsync(words[i], 0, sizeof(uint32_t), st));
         return set_error(HKB_ERR_TIMEOUT, "a kernel abandoned a bounded wait (status 0x%08x%s)", host[0] | host[1],
                          host[1] ? ", allocation-free entry point" : "");
     }

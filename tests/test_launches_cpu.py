@@ -1,0 +1,131 @@
+"""CPU tier: the host side of the launches against a stand-in CUDA runtime (fake_cudart.c): what a failing call leaves behind,
+what two host threads do to each other, which grid a problem gets.  Each check runs in a process of its own, this file as the
+program, with the stand-in preloaded."""
+import ctypes
+import os
+import shutil
+import subprocess
+import sys
+import threading
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+LIB = os.path.join(ROOT, "amd-kernels_b200", "kernels", "libhkb200.so")
+HKB_OK, HKB_ERR_CUDA = 0, -5
+i64 = ctypes.c_int64
+LAUNCH = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_char_p, ctypes.c_uint, ctypes.c_uint, ctypes.c_size_t, ctypes.c_int, ctypes.c_int,
+                          ctypes.POINTER(ctypes.c_void_p))
+CALL = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_char_p, ctypes.c_int)
+
+
+class Runtime:
+    """The stand-in's side of a check.  on_launch / on_limit / on_call may be replaced; what they return is what the call returns."""
+    def __init__(self):
+        self.fake = ctypes.CDLL(os.environ["LD_PRELOAD"])
+        self.lib = ctypes.CDLL(LIB)
+        self.lib.hkb_last_error.restype = self.lib.hkb_last_kernel.restype = ctypes.c_char_p
+        self.on_launch = lambda name, grid, smem, args: 0
+        self.on_limit = lambda name, value: 0
+        self.on_call = lambda name, value: 0
+        self._keep = (LAUNCH(lambda n, g, b, s, c, e, a: self.on_launch(n.decode(), g, s, a)),
+                      CALL(lambda n, v: self.on_limit(n.decode(), v)), CALL(lambda n, v: self.on_call(n.decode(), v)))
+        self.fake.fake_callbacks(*self._keep)
+
+    @staticmethod
+    def p(n=1):
+        return [ctypes.c_void_p((1 << 30) + (i << 33)) for i in range(n)]
+
+    def quant(self, M=64, K=512):
+        return self.lib.hkb_quant_fp8_per_token(*self.p(3), i64(M), i64(K), i64(K), None)
+
+    def pts(self, M, N, K, batch=1):
+        return self.lib.hkb_gemm_fp8_pts(*self.p(5), None, i64(batch), i64(M), i64(N), i64(K), None)
+
+    def blockscale(self, M, N, K):
+        return self.lib.hkb_gemm_fp8_blockscale(*self.p(5), i64(128), i64(M), i64(N), i64(K), None)
+
+    def mxfp4(self, M, N, K, batch=1):
+        return self.lib.hkb_gemm_mxfp4(*self.p(5), i64(batch), i64(M), i64(N), i64(K), None)
+
+    def mxfp4_tc(self, M, N, K, batch=1):
+        a, b, c, sa, sb = self.p(5)
+        return self.lib.hkb_gemm_mxfp4_tc(a, b, c, sa, 1, sb, 1, i64(batch), i64(M), i64(N), i64(K), None)
+
+    def mxfp4_static(self, M, N, K):
+        return self.lib.hkb_gemm_mxfp4_static(*self.p(5), i64(1), i64(M), i64(N), i64(K), None)
+
+    def ptgq(self, M, N, K):
+        return self.lib.hkb_gemm_fp8_ptgq(*self.p(4), None, i64(1), i64(M), i64(N), i64(K), None)
+
+    def moe_fp8(self, rows, N, K):
+        x, w, y, xs, ws, g, h, o, d = self.p(9)
+        return self.lib.hkb_moe_gemm_fp8_blockscale(x, w, y, xs, ws, None, g, h, o, d, i64(rows // 2), i64(rows), i64(8), i64(N), i64(K),
+                                                    i64(rows // 128 + 8), i64(2), None)
+
+    def moe_mxfp4(self, rows, N, K):
+        a, b, c, sa, sb, w, ids, ex = self.p(8)
+        return self.lib.hkb_moe_gemm_mxfp4(a, b, c, sa, sb, None, None, w, ids, ex, i64(rows // 2), i64(rows), i64(8), i64(N), i64(K),
+                                           i64(rows), i64(2), 1, None)
+
+    def calls(self):
+        """One call per kernel that is launched."""
+        return {"quantizer": self.quant, "per-token decode": lambda: self.pts(16, 4096, 1024), "per-token pairs": lambda: self.pts(4096, 8192, 512),
+                "per-token 64": lambda: self.pts(512, 1024, 512), "block-scale decode": lambda: self.blockscale(16, 4096, 1024),
+                "block-scale 128": lambda: self.blockscale(512, 1024, 512), "block-scale 256": lambda: self.blockscale(4096, 8192, 512),
+                "MXFP4 decode": lambda: self.mxfp4(16, 4096, 1024), "MXFP4 128": lambda: self.mxfp4(512, 1024, 512),
+                "MXFP4 192": lambda: self.mxfp4_tc(1000, 3080, 512), "MXFP4 pairs": lambda: self.mxfp4(4096, 8192, 512),
+                "MXFP4 static": lambda: self.mxfp4_static(256, 512, 512), "in-loop": lambda: self.ptgq(256, 512, 512),
+                "MoE FP8": lambda: self.moe_fp8(512, 1024, 512), "MoE MXFP4": lambda: self.moe_mxfp4(512, 1024, 512)}
+
+
+def check_failed_calls_leave_no_error_pending():
+    """A launch, an attribute, an allocation that fails is that call's error and nobody else's: the thread's pending error is taken
+    back, so that the next launch -- this library's or another's -- is not reported as failed."""
+    rt = Runtime()
+    for what, call in rt.calls().items():
+        assert call() == HKB_OK, (what, rt.lib.hkb_last_error())
+        failed = []
+
+        def fail_at(n):
+            seen = [0]
+
+            def hit(name, *_):
+                seen[0] += 1
+                if seen[0] == n:
+                    failed.append(name)
+                    return 701
+                return 0
+            return hit
+
+        for hook in ("on_launch", "on_limit", "on_call"):
+            for n in (1, 2, 3):
+                rt.lib.hkb_release()                     # scratch is allocated again
+                failed.clear()
+                setattr(rt, hook, fail_at(n))
+                rc = call()
+                setattr(rt, hook, lambda *_: 0)
+                if not failed:
+                    break
+                assert rc == HKB_ERR_CUDA, (what, hook, n, rc)
+                assert rt.fake.fake_pending() == 0, (what, hook, failed)
+                assert rt.quant() == HKB_OK and call() == HKB_OK, (what, hook, failed, rt.lib.hkb_last_error())
+
+
+def _run(check, tmp_path):
+    import pytest
+    inc = "/usr/local/cuda/include"
+    gcc = shutil.which("gcc")
+    if gcc is None or not os.path.exists(os.path.join(inc, "cuda_runtime_api.h")):
+        pytest.skip("no C compiler or CUDA runtime headers")
+    so = str(tmp_path / "fake_cudart.so")
+    src = os.path.join(ROOT, "tests", "fake_cudart.c")
+    subprocess.run([gcc, "-std=gnu11", "-O1", "-shared", "-fPIC", "-I", inc, src, "-o", so], check=True, capture_output=True, text=True)
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), check], env={**os.environ, "LD_PRELOAD": so}, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_failed_calls_leave_no_error_pending(tmp_path):
+    _run("check_failed_calls_leave_no_error_pending", tmp_path)
+
+
+if __name__ == "__main__":
+    globals()[sys.argv[1]]()

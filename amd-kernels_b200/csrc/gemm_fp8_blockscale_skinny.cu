@@ -310,7 +310,8 @@ gemm_fp8_blockscale_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const
 
 template <int NT>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB0, const CUtensorMap& tmB1, const BsSkinnyParams& p, int smem, int grid, cudaStream_t st) {
-    HKB_CUDA(cudaFuncSetAttribute(gemm_fp8_blockscale_skinny_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // the limit is the kernel's, not the call's: every call sets the same one, whatever its own size (calls may overlap)
+    HKB_CUDA(cudaFuncSetAttribute(gemm_fp8_blockscale_skinny_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     HKB_CUDA(launch_dependent(true, gemm_fp8_blockscale_skinny_kernel<NT>, grid, kThreads, smem, 0, st, tmA, tmB0, tmB1, p));
     return check_launch("gemm_fp8_blockscale_skinny_kernel");
 }

@@ -262,7 +262,8 @@ int launch_gemm_fp8_skinny(const void* A, const void* B, void* C, const float* s
     if (rc != HKB_OK) return rc;
     rc = make_tmap_bytes(&tmB1, B, (uint64_t)K, (uint64_t)N, 1, (uint32_t)maxw * 16);
     if (rc != HKB_OK) return rc;
-    HKB_CUDA(cudaFuncSetAttribute(gemm_fp8_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // the limit is the kernel's, not the call's: every call sets the same one, whatever its own size (calls may overlap)
+    HKB_CUDA(cudaFuncSetAttribute(gemm_fp8_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     const int grid = p.tiles < sms ? p.tiles : sms;
     HKB_CUDA(launch_dependent(true, gemm_fp8_skinny_kernel, grid, 192, smem, 0, st, tmA, tmB0, tmB1, p));
     return check_launch("gemm_fp8_skinny_kernel");

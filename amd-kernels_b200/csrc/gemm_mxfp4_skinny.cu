@@ -320,7 +320,8 @@ int launch_gemm_mxfp4_skinny(const void* A, const void* B, void* C, const void* 
     if (rc != HKB_OK) return rc;
     rc = make_tmap_bytes(&tmB16, B, (uint64_t)K / 2, (uint64_t)N, 1, 16);
     if (rc != HKB_OK) return rc;
-    HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // the limit is the kernel's, not the call's: every call sets the same one, whatever its own size (calls may overlap)
+    HKB_CUDA(cudaFuncSetAttribute(gemm_mxfp4_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     const int grid = p.tiles < sms ? p.tiles : sms;
     HKB_CUDA(launch_dependent(true, gemm_mxfp4_skinny_kernel, grid, 192 + 32 * kStagers, smem, 0, st, tmA, tmB128, tmB64, tmB16, p));
     return check_launch("gemm_mxfp4_skinny_kernel");

@@ -110,6 +110,37 @@ def check_failed_calls_leave_no_error_pending():
                 assert rt.quant() == HKB_OK and call() == HKB_OK, (what, hook, failed, rt.lib.hkb_last_error())
 
 
+def check_two_threads_do_not_take_each_others_shared_memory():
+    """The shared-memory limit belongs to the kernel, not to the call: a call of another shape from another thread, coming between
+    a call's setting it and its launch, must not make that launch ask for more than the limit allows."""
+    rt = Runtime()
+    limit, asked, between = {}, {}, []
+
+    def on_limit(name, value):
+        limit[name] = value
+        if between:
+            other = threading.Thread(target=lambda call: inner.append(call()), args=(between.pop(),))
+            other.start()
+            other.join()
+        return 0
+
+    def on_launch(name, grid, smem, args):
+        asked.setdefault(name, set()).add(smem)
+        return 0 if smem <= limit.get(name, 48 << 10) else 1                     # cudaErrorInvalidValue
+
+    rt.on_limit, rt.on_launch = on_limit, on_launch
+    shapes = [(M, N, K) for M in (1, 16, 32) for N, K in [(1024, 1024), (4096, 4096), (14336, 4096), (28672, 8192)]]
+    for kind in (rt.pts, rt.blockscale, rt.mxfp4):
+        for a in shapes:
+            for b in shapes:
+                inner = []
+                between[:] = [lambda: kind(*b)]
+                rc = kind(*a)
+                between.clear()
+                assert rc == HKB_OK and all(r == HKB_OK for r in inner), (rt.lib.hkb_last_kernel(), a, b, rt.lib.hkb_last_error())
+    assert sum(len(v) > 1 for v in asked.values()) >= 3, asked                    # decode kernels whose size depends on the shape
+
+
 def _run(check, tmp_path):
     import pytest
     inc = "/usr/local/cuda/include"
@@ -125,6 +156,10 @@ def _run(check, tmp_path):
 
 def test_failed_calls_leave_no_error_pending(tmp_path):
     _run("check_failed_calls_leave_no_error_pending", tmp_path)
+
+
+def test_two_threads_do_not_take_each_others_shared_memory(tmp_path):
+    _run("check_two_threads_do_not_take_each_others_shared_memory", tmp_path)
 
 
 if __name__ == "__main__":

@@ -720,8 +720,6 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
     p.m_blks = (int)((M + BM - 1) / BM);
     const int sms = sm_count();
     HKB_REQUIRE(sms > 0, HKB_ERR_CUDA, "no CUDA device");
-    const int bn = mxfp4_tile_width(p.m_blks, N, batch, sms, false);
-    p.n_blks = (int)((N + bn - 1) / bn);
     p.sfa_rblks = sf_tc_rblks(M);
     p.sfb_rblks = sf_tc_rblks(N);
     p.katoms = sf_tc_katoms(K);
@@ -750,10 +748,13 @@ int gemm_mxfp4_impl(const void* A, const void* B, void* C, const void* sfa, cons
         return launch_gemm_mxfp4_skinny(A, B, C, sfa, sfb, sfa_tc, sfb_tc, c_a, c_b, M, N, K, p.status, st);
     }
 
-    // CTA pairs on 256 x 192 tiles when there are two waves of one-CTA tiles (HKB_MXFP4_PAIRS=0: never)
+    // CTA pairs on 256 x 192 tiles when there are two waves of one-CTA tiles of that width (HKB_MXFP4_PAIRS=0: never); the
+    // split-cat store lives in the one-CTA kernels, whose width has a rule of its own.
     static const bool pairs_on = [] { const char* v = getenv("HKB_MXFP4_PAIRS"); return !(v && v[0] == '0'); }();
-    const int64_t pair_tiles = ((M + 255) / 256) * ((N + 191) / 192) * batch;
-    const bool pair = pairs_on && (int64_t)p.m_blks * ((N + 191) / 192) * batch >= 2LL * sms && M > 128 && pair_tiles >= sms / 2 && sms >= 2 && !sc;     // the split-cat store lives in the one-CTA kernels
+    const int64_t n_blks192 = (N + 191) / 192, pair_tiles = ((M + 255) / 256) * n_blks192 * batch;
+    const bool pair = pairs_on && p.m_blks * n_blks192 * batch >= 2LL * sms && M > 128 && pair_tiles >= sms / 2 && sms >= 2 && !sc;
+    const int bn = pair ? PairCfg::BN : mxfp4_tile_width(p.m_blks, N, batch, sms, false);
+    p.n_blks = (int)((N + bn - 1) / bn);
 
     const size_t sfa_bytes = (size_t)batch * p.sfa_rblks * p.katoms * 512;
     const size_t sfb_bytes = (size_t)batch * p.sfb_rblks * p.katoms * 512;

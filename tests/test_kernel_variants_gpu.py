@@ -42,6 +42,30 @@ def test_mxfp4_mul_add_and_tile_width_rule(hk, shape, kernel):
     _check(C, gemm.mul_add(gemm.gemm_mxfp4(ac, wc, asc, wsc), c_a, c_b), f"mxfp4 mul_add {shape}")
 
 
+@pytest.mark.parametrize("batch,M,N,mul_add", [(1, 3456, 4096, False), (1, 3400, 4096, True), (3, 1152, 4096, False)])
+def test_mxfp4_pairs_where_one_cta_tiles_would_be_narrow(hk, batch, M, N, mul_add):
+    """CTA pairs at sizes for which the width rule of the one-CTA kernels says 128: the pairs walk their own 192-wide tiles."""
+    K = 384
+    ac, wc, asc, wsc = _mxfp4_operands(M, N, K, batch=batch)
+    C = torch.full((batch, M, N) if batch > 1 else (M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    if mul_add:
+        g = torch.Generator().manual_seed(3)
+        c_a, c_b = torch.randn(M, N, generator=g).bfloat16(), torch.randn(M, N, generator=g).bfloat16()
+        hk.fused_gemm.afp4wfp4_mul_add.dispatch(_dev(ac), _dev(wc), C, _dev(asc), _dev(wsc), _dev(c_a), _dev(c_b))
+        ref = gemm.mul_add(gemm.gemm_mxfp4(ac, wc, asc, wsc), c_a, c_b)
+    elif batch > 1:
+        hk.batched_gemm.afp4wfp4.dispatch(_dev(ac), _dev(wc), C, _dev(asc), _dev(wsc))
+        ref = [gemm.gemm_mxfp4(ac[b], wc[b], asc[b], wsc[b]) for b in range(batch)]
+    else:
+        hk.gemm.afp4wfp4.dispatch(_dev(ac), _dev(wc), C, _dev(asc), _dev(wsc))
+        ref = gemm.gemm_mxfp4(ac, wc, asc, wsc)
+    torch.cuda.synchronize()
+    assert hk.last_kernel() == "gemm_mxfp4_pair_kernel<256x192>"
+    _status_ok()
+    for c, r in zip(C, ref) if batch > 1 else [(C, ref)]:
+        _check(c, r, f"mxfp4 pairs {batch}x{M}x{N}")
+
+
 @pytest.mark.parametrize("shape", [(1, 16, 128), (7, 2000, 384), (16, 10064, 256), (33, 17600, 128), (64, 9488, 1152), (64, 36000, 256)])
 def test_mxfp4_skinny_kernel(hk, shape):
     """Tile widths of 1 to 15 units, one and two rounds, an odd number of K atoms, both layouts of either scale array."""

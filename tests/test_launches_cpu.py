@@ -141,6 +141,36 @@ def check_two_threads_do_not_take_each_others_shared_memory():
     assert sum(len(v) > 1 for v in asked.values()) >= 3, asked                    # decode kernels whose size depends on the shape
 
 
+def check_mxfp4_tiles_cover_the_result_once():
+    """The row and column tile counts that an MXFP4 kernel walks are those of its own tile, and no cluster or block is left
+    without one: a count for another width leaves columns out or walks tiles that lie wholly past N."""
+    rt = Runtime()
+    tiles = {"gemm_mxfp4_pair_kernel<256x192>": (256, 192, 2), "gemm_mxfp4_kernel<192>": (128, 192, 1), "gemm_mxfp4_kernel<128>": (128, 128, 1)}
+    launched = []
+
+    def on_launch(name, grid, smem, args):
+        if "gemm_mxfp4" in name:
+            p = 4 if "pair" in name else 2                                       # behind the tensor maps: M, N, K, batch, m_blks, n_blks
+            launched.append((grid, ctypes.cast(args[p], ctypes.POINTER(ctypes.c_int))[:6]))
+        return 0
+
+    rt.on_launch = on_launch
+    seen = set()
+    for batch in (1, 3):
+        for M in [100, 129, 300] + list(range(640, 8193, 64 if batch == 1 else 640)):
+            for N in [8, 136, 1000] + list(range(1024, 28673, 512 if batch == 1 else 1920)):
+                launched.clear()
+                assert rt.mxfp4_tc(M, N, 1024, batch) == HKB_OK, rt.lib.hkb_last_error()
+                kernel = rt.lib.hkb_last_kernel().decode()
+                seen.add(kernel)
+                bm, bn, ctas = tiles[kernel]
+                (grid, got), = launched
+                want = [M, N, 1024, batch, -(-M // bm), -(-N // bn)]
+                assert got == want, (kernel, got, want)
+                assert grid == ctas * min(148 // ctas, batch * want[4] * want[5]), (kernel, grid, want)
+    assert seen == set(tiles), seen
+
+
 def _run(check, tmp_path):
     import pytest
     inc = "/usr/local/cuda/include"
@@ -160,6 +190,10 @@ def test_failed_calls_leave_no_error_pending(tmp_path):
 
 def test_two_threads_do_not_take_each_others_shared_memory(tmp_path):
     _run("check_two_threads_do_not_take_each_others_shared_memory", tmp_path)
+
+
+def test_mxfp4_tiles_cover_the_result_once(tmp_path):
+    _run("check_mxfp4_tiles_cover_the_result_once", tmp_path)
 
 
 if __name__ == "__main__":

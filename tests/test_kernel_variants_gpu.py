@@ -3,7 +3,8 @@ import pytest
 import torch
 
 from oracle import gemm
-from test_gemm_gpu import DEV, _check, _dev, _fp8_operands, _mxfp4_operands, _status_ok
+from test_gemm_gpu import (DEV, _check, _dev, _fp8_operands, _moe_call, _moe_mxfp4_call, _moe_mxfp4_routing, _mxfp4_operands,
+                           _routing, _status_ok)
 
 pytestmark = pytest.mark.gpu
 
@@ -120,6 +121,29 @@ def test_blockscale_skinny_kernel(hk, shape):
     assert torch.equal(C, big[:M]) and torch.equal(C_ma, big_ma[:M])
 
 
+@pytest.mark.parametrize("shape", [(1, 128, 128), (17, 2560, 640), (32, 14336, 256)])
+def test_blockscale_skinny_pitched_result(hk, shape):
+    """One destination with a row pitch: the column slab of a wider matrix, nothing outside it touched."""
+    M, N, K = shape
+    aq, bq, _, _ = _fp8_operands(M, N, K, seed=51)
+    g = torch.Generator().manual_seed(7)
+    sa = torch.rand(M, K // 128, generator=g) * 0.1 + 0.01
+    sb = torch.rand(K // 128, N // 128, generator=g) * 0.1 + 0.01
+    a, b, sad, sbd = _dev(aq), _dev(bq), sa.to(DEV), sb.to(DEV)
+    plain = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    hk.gemm.a8w8_blockscale.dispatch(a, b, plain, sad, sbd)
+    ldc, col0 = 2 * N + 48, N + 32
+    out = torch.full((M + 1, ldc), 7.0, dtype=torch.bfloat16, device=DEV)
+    hk.gemm.a8w8_blockscale.dispatch_scatter(a, b, [out.data_ptr() + col0 * 2], ldc, sad, sbd)
+    assert hk.last_kernel() == "gemm_fp8_blockscale_skinny_kernel"
+    torch.cuda.synchronize()
+    _status_ok()
+    _check(plain, gemm.gemm_fp8_blockscale(aq, bq, sa, sb), f"blockscale skinny {shape}")
+    assert torch.equal(out[:M, col0:col0 + N], plain)
+    out[:M, col0:col0 + N] = 7.0
+    assert bool((out == 7.0).all())
+
+
 def test_shim_reads_tensors_parameters_and_subclasses_alike(hk):
     """Plain tensors and Parameters go through the native reads, subclasses through the general ones: same results, same
     refusals, on the current stream of the tensors' device."""
@@ -166,43 +190,102 @@ def test_per_token_pairs_split_last_wave(hk, batch, M, N, K, with_bias):
     _check(C, gemm.gemm_fp8_per_token(aq, bq, sa, sb, bias), f"per-token pairs {batch}x{M}x{N}x{K}")
 
 
-@pytest.mark.parametrize("M", [16, 300])
-def test_dependent_launches_under_graph_capture(hk, M):
-    """Quantizer and GEMMs captured as one chain of programmatic launches: replays follow the inputs, kernel after kernel."""
-    N, K = 5120, 1024
-    g = torch.Generator().manual_seed(M)
-    w = (torch.randn(N, K, generator=g) * 0.02).bfloat16().to(DEV)
-    x = torch.zeros(M, K, dtype=torch.bfloat16, device=DEV)
+def _chained_layers(hk, M, N, K, g):
+    """Layers as (quantize(x, operands), new operands, gemm(operands, C), C's shape), weights quantized."""
+    E, N_moe = 4, 1024
     mod = hk.gemm.afp4wfp4
     u8 = lambda *s: torch.zeros(*s, dtype=torch.uint8, device=DEV)      # noqa: E731
     f32 = lambda *s: torch.zeros(*s, device=DEV)                         # noqa: E731
-    wq, ws, xq, xs = u8(N, K), f32(N, 1), u8(M, K), f32(M, 1)
-    bq, bs, yq, ys = u8(N, K), f32(K // 128, N // 128), u8(M, K), f32(M, K // 128)
-    fq, fs, zq, zs = u8(N, K // 2), u8(mod.sf_tc_bytes(1, N, K)), u8(M, K // 2), u8(mod.sf_tc_bytes(1, M, K))
+    w = (torch.randn(N, K, generator=g) * 0.02).bfloat16().to(DEV)
+    wq, ws, bq, bs, fq, fs, ft = u8(N, K), f32(N, 1), u8(N, K), f32(K // 128, N // 128), u8(N, K // 2), u8(N, K // 32), u8(mod.sf_tc_bytes(1, N, K))
     hk.per_token_quant_fwd(w, wq, ws)
     hk.weight_quant_128x128(w, bq, bs)
-    hk.fused_rmsnorm_mxfp4_quant_tc_fwd(w, None, fq, None, fs, 1e-6)
-    C = [torch.zeros(M, N, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+    hk.fused_rmsnorm_mxfp4_quant_fwd(w, None, fq, fs, 1e-6)
+    mod.sf_to_tc(fs, ft, K)
+    eq, es = u8(E, N_moe, K), f32(E, K // 128, N_moe // 128)
+    eq4, es4 = u8(E, N_moe, K // 2), u8(E, N_moe, K // 32)
+    for e in range(E):
+        we = (torch.randn(N_moe, K, generator=g) * 0.02).bfloat16().to(DEV)
+        hk.weight_quant_128x128(we, eq[e], es[e])
+        hk.fused_rmsnorm_mxfp4_quant_fwd(we, None, eq4[e], es4[e], 1e-6)
+    hist, offs, gather, data = (_dev(v) for v in _routing(M, E, 2, seed=5))
+    ids, eids, gate, total = _moe_mxfp4_routing(M, E, 2, seed=6)
+    ids, eids, gate, one = _dev(ids), _dev(eids), _dev(gate), torch.ones(1, device=DEV)
+    fp8_1x128 = lambda x, o: hk.fused_rmsnorm_fp8_quant_fwd(x, None, *o, 1e-6)      # noqa: E731
+    mxfp4 = lambda x, o: hk.fused_rmsnorm_mxfp4_quant_fwd(x, None, *o, 1e-6)        # noqa: E731
+    return [
+        (lambda x, o: hk.per_token_quant_fwd(x, *o), lambda: (u8(M, K), f32(M, 1)),
+         lambda o, C: hk.gemm.a8w8_per_token.dispatch(o[0], wq, C, o[1], ws), (M, N)),
+        (fp8_1x128, lambda: (u8(M, K), f32(M, K // 128)), lambda o, C: hk.gemm.a8w8_blockscale.dispatch(o[0], bq, C, o[1], bs), (M, N)),
+        (lambda x, o: hk.fused_rmsnorm_mxfp4_quant_tc_fwd(x, None, o[0], None, o[1], 1e-6), lambda: (u8(M, K // 2), u8(mod.sf_tc_bytes(1, M, K))),
+         lambda o, C: mod.dispatch_tc(o[0], fq, C, o[1], ft, True, True), (M, N)),
+        (mxfp4, lambda: (u8(M, K // 2), u8(M, K // 32)), lambda o, C: mod.dispatch(o[0], fq, C, o[1], fs), (M, N)),
+        (fp8_1x128, lambda: (u8(M, K), f32(M, K // 128)),
+         lambda o, C: _moe_call(hk, o[0], eq, C, o[1], es, None, gather, hist, offs, data, 2), (2 * M, N_moe)),
+        (mxfp4, lambda: (u8(M, K // 2), u8(M, K // 32)),
+         lambda o, C: _moe_mxfp4_call(hk, o[0], eq4, C, o[1], es4, one, one.expand(E).contiguous(), gate, ids, eids, total, 2, True), (2 * M, N_moe)),
+    ]
 
-    def chain():
-        hk.per_token_quant_fwd(x, xq, xs)
-        hk.gemm.a8w8_per_token.dispatch(xq, wq, C[0], xs, ws)
-        hk.fused_rmsnorm_fp8_quant_fwd(x, None, yq, ys, 1e-6)
-        hk.gemm.a8w8_blockscale.dispatch(yq, bq, C[1], ys, bs)
-        hk.fused_rmsnorm_mxfp4_quant_tc_fwd(x, None, zq, None, zs, 1e-6)
-        mod.dispatch_tc(zq, fq, C[2], zs, fs, True, True)
 
-    chain()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
-        chain()
-    for seed in range(8):
-        x.copy_(torch.randn(M, K, generator=torch.Generator().manual_seed(seed)).bfloat16())
-        chain()
-        want = [c.clone() for c in C]
+@pytest.mark.parametrize("M,N", [(16, 5120), (300, 5120), (300, 25600)])      # the last one takes the CTA-pair kernels
+def test_dependent_launches_under_graph_capture(hk, M, N):
+    """Quantizers, pre-passes and GEMMs issued without a wait, eagerly and as a captured chain of programmatic launches, give
+    what the same calls give one at a time.  Every layer runs for two inputs in a row (the second rewrites the scratch that the first
+    one's GEMM reads), and codes, scales and scratch hold another input's values when a chain starts, so a kernel
+    that ran ahead of the one before it would show."""
+    K = 1024
+    layers = _chained_layers(hk, M, N, K, torch.Generator().manual_seed(M))
+    x = [torch.zeros(M, K, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    operands = [[new() for _ in x] for _, new, _, _ in layers]
+    C = [[torch.zeros(shape, dtype=torch.bfloat16, device=DEV) for _ in x] for _, _, _, shape in layers]
+
+    def chain(wait=lambda: None, quantizers=True):
+        for (quantize, _, multiply, _), ops, c in zip(layers, operands, C):
+            for i in (1, 0):
+                if quantizers:
+                    quantize(x[i], ops[i])
+                wait()
+            for i in (0, 1):
+                multiply(ops[i], c[i])
+                wait()
+
+    def fill(seed):
+        for i in range(2):
+            x[i].copy_(torch.randn(M, K, generator=torch.Generator().manual_seed(2 * seed + i)).bfloat16())
+
+    def poison(seed):
+        fill(100 + seed)
+        chain(torch.cuda.synchronize)
         for c in C:
-            c.fill_(float("nan"))
-        graph.replay()
+            for t in c:
+                t.fill_(float("nan"))
+        fill(seed)
         torch.cuda.synchronize()
-        assert all(torch.equal(c, v) for c, v in zip(C, want)) and want[0].abs().max() > 0
+
+    def same(want):
+        torch.cuda.synchronize()
+        return [torch.equal(t, v) for c, w in zip(C, want) for t, v in zip(c, w)]
+
+    chain(torch.cuda.synchronize)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        chain()                                                  # scratch is kept per stream and has to exist before a capture
+    side.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        chain()
+    for seed in range(4):
+        fill(seed)
+        chain(torch.cuda.synchronize)
+        want = [[t.clone() for t in c] for c in C]
+        assert all(t.abs().max() > 0 and bool(t.isfinite().all()) for w in want for t in w)
+        poison(seed)
+        chain(quantizers=False)
+        assert not any(same(want))                               # what stale operands would give
+        poison(seed)
+        chain()
+        assert all(same(want))
+        poison(seed)
+        graph.replay()
+        assert all(same(want))
     _status_ok()

@@ -45,8 +45,9 @@ inline int check_launch(const char* what) {
 
 // Launch whose grid may start before the kernel ahead of it in the stream has ended (programmatic dependent launch): its
 // blocks set up barriers, tensor memory and descriptors meanwhile.  EVERY thread of such a kernel calls pdl_wait() before
-// its first access to global memory -- operands, results, scratch -- so that all earlier work has completed and is visible;
-// that also keeps the chain whole when the next kernel is launched this way in turn.  cluster: CTAs per cluster, 0 = none.
+// its first read or write of global memory -- operands, results, scratch -- so that all earlier work has completed and is
+// visible; that also keeps the chain whole when the next kernel is launched this way in turn.  Only an L2 prefetch, which
+// hands no value to the kernel, may come before it (tma_prefetch_3d).  cluster: CTAs per cluster, 0 = none.
 // early = false: an ordinary launch of the same kernel.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent(bool early, void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, unsigned cluster, cudaStream_t st, Args&&... args) {

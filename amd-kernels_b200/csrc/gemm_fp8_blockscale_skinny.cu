@@ -12,10 +12,10 @@
 //    128-row scale groups: each thread picks its row's group.
 //  * Staging warps transpose the activation scales, eight K blocks at a time, into shared memory ([K block][token]), where
 //    the epilogue reads them as broadcasts.
-//  * What bounds it now is the MMA thread and the hand-off, at about 0.3 us per K block and tile with one K block per
+//  * What bounds it is the MMA thread and the hand-off, at about 0.3 us per K block and tile with one K block per
 //    stage and two commits for each.  So a stage holds two K blocks, one commit publishes both partial products, and the
-//    epilogue returns the operands: 24 x 14336 x 4096 took 18.0 us before that and 16.2 with it (four instead of eight
-//    epilogue warps: 20.3; the MMAs of two K blocks interleaved: no change).
+//    epilogue returns the operands: 24 x 14336 x 4096 takes 16.2 us, 18.0 with one K block per stage (and 20.3 with four
+//    instead of eight epilogue warps; the MMAs of two K blocks interleaved: no difference).
 //
 // Every K block is promoted in order with the same fused multiply-adds as in the large kernel, so the two give the same
 // bits.  Cold L2, us, large kernel / this one: 24 x 14336 x 4096 24.8 / 16.2, 32 x 28672 x 8192 53.8 / 44.7 (5.3 TB/s),

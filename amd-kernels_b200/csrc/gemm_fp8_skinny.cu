@@ -16,8 +16,8 @@
 //    K blocks, so the SMs do not pull the same byte columns of the weight rows in lockstep.
 //
 //  * Ahead of the quantizer's end.  The first ring of weight tiles is prefetched into L2 before the
-//    kernel waits for the kernel ahead of it (16 x 28672 x 8192, quantizer + GEMM: 47.2 us a pass
-//    before, 46.2 with it; the MXFP4 and block-scale decode kernels did not gain from the same).
+//    kernel waits for the kernel ahead of it (16 x 28672 x 8192, quantizer + GEMM: 46.2 us a pass,
+//    47.2 without; the MXFP4 and block-scale decode kernels did not gain from the same).
 //
 // A tile of w units is staged with one TMA box of exactly its rows (two tensor maps: base and
 // base + 1 units) and multiplied by one tcgen05.mma of N = 16 w (the instruction descriptor is built per
@@ -101,7 +101,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     if (warp == 0 && blockIdx.x < p.tiles && elect_one())
         for (int i = 0; i < min(p.stages, kblocks); ++i) tma_prefetch_3d(blockIdx.x < p.rem ? &tmB1 : &tmB0, (kb0 + i) % kblocks * 128, TILE_COL0((int)blockIdx.x), 0);
     __syncwarp();
-    pdl_wait();      // nothing in global memory is touched before this
+    pdl_wait();      // nothing in global memory is read or written before this; the prefetch above is a hint to L2 only
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

@@ -79,8 +79,8 @@ struct GatherJob {
 // All that has to move before the GEMM, in one launch: A's scales, B's scales, the MoE row gather.  Latency bounds it
 // (a few MB at most), so a block is small -- 128 rows x 8 atoms, 4 KB through shared memory, one 16-byte load and one
 // 16-byte store per thread -- and the three jobs run side by side instead of as three launches.  M = 1000, N = 3080,
-// K = 4224: 22.4 us in two launches of 128 x 32-atom blocks before, 3.7 now; 1024 sorted rows and 8 experts
-// of 8192 x 8192: 27.2 us in three launches before, 10.6 now.
+// K = 4224: 3.7 us, as two launches of 128 x 32-atom blocks 22.4; 1024 sorted rows and 8 experts of 8192 x 8192: 10.6 us,
+// as three launches 27.2.
 __global__ void __launch_bounds__(256)
 mxfp4_prepass_kernel(const SfJob ja, const SfJob jb, const GatherJob jg) {
     constexpr int kPitch = 132;                            // words per atom in shared memory: 128 + 4, keeps 16-byte alignment
@@ -168,7 +168,7 @@ struct Cfg {
 // c_a / c_b of 32 consecutive columns of one row, for the fused multiply-add epilogue.  All eight 16-byte loads of a
 // chunk go out together, one chunk ahead of its use (the first before the accumulator is waited for), behind an L2
 // prefetch of the tile's whole row: loaded where they were used, four round trips to HBM per chunk one after the other,
-// they took more of a tile's time than its main loop (M = 1000, N = 3080, K = 4224: 34.5 us before, 21.4 now with the same 128-wide tiles).
+// they take more of a tile's time than its main loop (M = 1000, N = 3080, K = 4224 on 128-wide tiles: 34.5 us so, 21.4 like this).
 struct MulAddChunk {
     uint4 a[4], b[4];
     __device__ __forceinline__ void fetch(const Mxfp4Params& p, int64_t row_off, int col0, bool row_ok) {

@@ -34,11 +34,11 @@ struct TView {
 
 [[noreturn]] void fail(const std::string& m) { throw std::runtime_error(m); }
 
-// What a call needs from torch, looked up once: a pass of two calls spent about 30 us on the host, most of it in
-// attribute names built as strings, dtype reprs, a Python context manager and a Stream object per call.  Plain tensors (exactly
-// torch.Tensor or Parameter) are read through interned names and torch._C's own functions instead; everything else --
-// subclasses, duck-typed objects -- keeps the general path below.  Held for the life of the process, under the GIL.
-// 128 x 1024 x 1024, quantizer + GEMM: 29.7 us a pass before, 13.6 now; row-major MXFP4 with multiply-add 35.7 / 28.7.
+// What a call needs from torch, looked up once: through the general path below a pass of two calls spends about 30 us on
+// the host, most of it in attribute names built as strings, dtype reprs, a Python context manager and a Stream object per call.
+// Plain tensors (exactly torch.Tensor or Parameter) are read through interned names and torch._C's own functions instead;
+// everything else -- subclasses, duck-typed objects -- keeps the general path.  Held for the life of the process, under the GIL.
+// A pass of quantizer + GEMM, general path / this: 128 x 1024 x 1024 29.7 / 13.6 us, row-major MXFP4 with multiply-add 35.7 / 28.7.
 struct Torch {
     PyObject *data_ptr, *shape, *dtype, *is_contiguous, *is_cuda, *get_device;      // interned attribute names
     PyObject *tensor, *parameter;                                                   // types

@@ -182,7 +182,8 @@ int hkb_gemm_fp8_blockscale_mul_add(const void* A, const void* B, void* C, const
  * may overlap on the GPU (up to 8 streams per device keep their own scratch; beyond that the least
  * recently used stream's scratch is recycled behind a device-wide synchronisation).  A call that
  * has to allocate or grow its stream's scratch calls cudaMalloc / cudaFree, so the first call of a
- * size on a stream must come before any stream capture.  Replaces
+ * size on a stream must come before any stream capture.  (Decode calls -- batch 1, M <= 64,
+ * N % 16 == 0, C 32-byte aligned -- read the scales as they are and use no scratch.)  Replaces
  *   gemm_afp4wfp4_tk.dispatch           kernels/gemm-basic/gemm_afp4wfp4/kernel.cpp:1-12,48-159
  *   batched_gemm_afp4wfp4_tk.dispatch   kernels/gemm-batched/batched_gemm_afp4wfp4/kernel.cpp:3-7,52-168
  * (operand spec from those files' header comments; the reference kernels themselves take

@@ -187,6 +187,10 @@ gemm_fp8_blockscale_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const
             const bool warp_has_rows = quarter * 32 < rows;              // warp-uniform
             const int n = n0 + (row_ok ? row_in_tile : 0);
             const int group = (n >> 7) - (n0 >> 7);                      // 0 or 1
+            if (p.c_a && warp_has_rows && col0 + (lane & (NC - 1)) < p.M) {      // this warp's part of c_a and c_b, into L2
+                const int64_t off = (int64_t)(col0 + (lane & (NC - 1))) * p.N + n0 + quarter * 32;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"((lane < 16 ? p.c_a : p.c_b) + off));
+            }
             float2 acc2[NC / 2];
 #pragma unroll
             for (int j = 0; j < NC / 2; ++j) acc2[j] = make_float2(0.0f, 0.0f);
@@ -241,15 +245,25 @@ gemm_fp8_blockscale_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const
                 if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
             }
             if (ok && row_ok) {
+                float v[NC];
 #pragma unroll
-                for (int j = 0; j < NC; ++j) {
-                    const int64_t m = col0 + j;
-                    if (m < p.M) {
-                        float v = (j & 1) ? acc2[j / 2].y : acc2[j / 2].x;
-                        if (p.c_a) v = __fmaf_rn(__bfloat162float(p.c_a[m * p.N + n]), v, __bfloat162float(p.c_b[m * p.N + n]));
-                        p.C[m * p.ldc + n] = __float2bfloat16_rn(v);
+                for (int j = 0; j < NC; ++j) v[j] = (j & 1) ? acc2[j / 2].y : acc2[j / 2].x;
+                if (p.c_a) {
+                    // All loads go out before the first store: C may be c_a or c_b, so the compiler cannot move them up, and one
+                    // round trip per token is longer than the whole K loop of a small layer.
+                    __nv_bfloat16 ca[NC], cb[NC];
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) {
+                        const int64_t off = (int64_t)min(col0 + j, p.M - 1) * p.N + n;
+                        ca[j] = p.c_a[off];
+                        cb[j] = p.c_b[off];
                     }
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) v[j] = __fmaf_rn(__bfloat162float(ca[j]), v[j], __bfloat162float(cb[j]));
                 }
+#pragma unroll
+                for (int j = 0; j < NC; ++j)
+                    if (col0 + j < p.M) p.C[(int64_t)(col0 + j) * p.ldc + n] = __float2bfloat16_rn(v[j]);
             }
         }
     } else {

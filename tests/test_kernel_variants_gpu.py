@@ -174,7 +174,11 @@ def test_shim_reads_tensors_parameters_and_subclasses_alike(hk):
 
 @pytest.mark.parametrize("batch,M,N,K,with_bias", [(8, 512, 4096, 128, True), (1, 2300, 6408, 256, False), (2, 1290, 5000, 384, True)])
 def test_per_token_pairs_split_last_wave(hk, batch, M, N, K, with_bias):
-    """256 x 256 tiles whose last wave is mostly empty and walked as halves; rows, columns and halves past the edges."""
+    """256 x 256 tiles whose last wave is mostly empty and walked as halves (that they are is shown on the CPU, test_launches_cpu.py);
+    rows, columns and halves past the edges."""
+    tiles, clusters = batch * -(-M // 256) * -(-N // 256), torch.cuda.get_device_properties(0).multi_processor_count // 2
+    if not (tiles > clusters and 0 < 2 * (tiles % clusters) <= clusters):
+        pytest.skip(f"{tiles} tiles on {clusters} clusters leave no small last wave")
     aq, bq, sa, sb = _fp8_operands(M, N, K, batch)
     bias = torch.randn(batch, N, generator=torch.Generator().manual_seed(2)).bfloat16() if with_bias else None
     C = torch.full((batch, M, N) if batch > 1 else (M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
@@ -184,8 +188,6 @@ def test_per_token_pairs_split_last_wave(hk, batch, M, N, K, with_bias):
         hk.gemm.a8w8_per_token.dispatch(_dev(aq), _dev(bq), C, _dev(sa), _dev(sb))
     torch.cuda.synchronize()
     assert hk.last_kernel() == "gemm_fp8_kernel<256,pts,pair>"
-    tiles, clusters = batch * -(-M // 256) * -(-N // 256), torch.cuda.get_device_properties(0).multi_processor_count // 2
-    assert tiles > clusters and 0 < 2 * (tiles % clusters) <= clusters or clusters != 74
     _status_ok()
     _check(C, gemm.gemm_fp8_per_token(aq, bq, sa, sb, bias), f"per-token pairs {batch}x{M}x{N}x{K}")
 

@@ -171,6 +171,41 @@ def check_mxfp4_tiles_cover_the_result_once():
     assert seen == set(tiles), seen
 
 
+class GemmParams(ctypes.Structure):
+    """The FP8 GEMM kernels' parameters (csrc/gemm_fp8.cu) up to the field that is read here."""
+    _fields_ = ([(n, ctypes.c_int) for n in "M N K batch m_blks n_blks a_box_rows".split()] + [(n, ctypes.c_void_p) for n in "sa sb bias C".split()] +
+                [("gn", ctypes.c_int), ("c_a", ctypes.c_void_p), ("c_b", ctypes.c_void_p), ("ldc", i64), ("peer", ctypes.c_void_p * 7), ("n_peer", ctypes.c_int)] +
+                [(n, ctypes.c_void_p) for n in "expt_data expt_hist expt_offs bias_f32 c2".split()] +
+                [(n, ctypes.c_int) for n in "sc_s1 sc_s2 sc_s3 group_m split_from".split()])
+
+
+def check_per_token_pairs_split_a_small_last_wave():
+    """What the CTA-pair kernel is told to walk: 256 x 256 tiles over 74 clusters, those of a last wave that fills at most half of
+    the clusters as two halves each, everything else whole."""
+    rt = Runtime()
+    launched = []
+
+    def on_launch(name, grid, smem, args):
+        p = GemmParams.from_address(args[2])
+        launched.append((grid, p.M, p.N, p.K, p.batch, p.m_blks, p.n_blks, p.group_m, p.split_from))
+        return 0
+
+    rt.on_launch = on_launch
+    split = whole = 0
+    for batch, M, N in [(8, 512, 4096), (2, 1290, 5000), (1, 2300, 6408)] + [(1, M, N) for M in range(1024, 8193, 640) for N in range(2048, 16385, 1024)]:
+        launched.clear()
+        assert rt.pts(M, N, 256, batch) == HKB_OK, rt.lib.hkb_last_error()
+        if rt.lib.hkb_last_kernel() != b"gemm_fp8_kernel<256,pts,pair>":
+            continue
+        mb, nb = -(-M // 256), -(-N // 256)
+        tiles = batch * mb * nb
+        tail = tiles % 74 if tiles > 74 else 0
+        want = tiles - tail if 0 < tail <= 37 else tiles
+        assert launched == [(2 * min(74, tiles), M, N, 256, batch, mb, nb, 8, want)], (launched, want)
+        split, whole = split + (want < tiles), whole + (want == tiles)
+    assert split > 20 and whole > 20, (split, whole)
+
+
 def _run(check, tmp_path):
     import pytest
     inc = "/usr/local/cuda/include"
@@ -194,6 +229,10 @@ def test_two_threads_do_not_take_each_others_shared_memory(tmp_path):
 
 def test_mxfp4_tiles_cover_the_result_once(tmp_path):
     _run("check_mxfp4_tiles_cover_the_result_once", tmp_path)
+
+
+def test_per_token_pairs_split_a_small_last_wave(tmp_path):
+    _run("check_per_token_pairs_split_a_small_last_wave", tmp_path)
 
 
 if __name__ == "__main__":

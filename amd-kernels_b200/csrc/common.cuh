@@ -74,8 +74,14 @@ cudaError_t launch_dependent(bool early, void (*kern)(KArgs...), unsigned grid, 
 
 // Whether a persistent GEMM starts early.  Blocks that start early land on the SMs in the order in which the quantizer
 // leaves them, which costs the long kernels some of the L2 sharing between neighbouring tiles, and a launch latency is
-// nothing to them: 16384 x 57344 x 8192 block-scale took 8.71 ms a pass early and 8.54 not, 4096 x 14336 x 4096 (12 tiles per
-// block) 310 us against 305; at 3.5 tiles per pair (8 x 512 x 4096 x 4096 per-token) 83.2 us early and 84.1 not.
+// nothing to them: 16384 x 57344 x 8192 block-scale takes 8.71 ms a pass early and 8.54 not, 4096 x 14336 x 4096 (12 tiles per
+// block) 310 us and 305.  Up to four tiles per block the start saves 0.5 to 2 us a pass.  Early / not, us a pass of quantizer +
+// GEMM in a replayed graph: per-token 512 x 4096 x 4096 20.3 / 21.1, 2000 x 3000 x 4096 (2.6 tiles per block) 34.8 / 35.8,
+// 8 x 512 x 4096 x 4096 (3.5) 65.9 / 66.9; block-scale 512 x 14336 x 4096 (3.0) 55.7 / 56.6, 4096 x 4096 x 4096 (3.5)
+// 88.5 / 89.7, 1024 x 14336 x 7168 (3.0) 131.8 / 133.4, 4608 x 4096 x 7168 (3.9) 153.3 / 152.9; MXFP4 1024 x 4096 x 4096 16.7 /
+// 17.4, 2048 x 4096 x 4096 25.2 / 25.8.  Of 40 such sizes between two and four tiles, two were behind by less than 0.5 us.
+// Grouped block-scale sits on the line where K is long: 2048 tokens, top-2 of 8, N = 3072: K = 1024 34.5 / 35.2, K = 4096
+// 81.0 / 79.9.
 inline bool starts_early(int64_t tiles, int64_t workers) { return tiles <= 4 * workers; }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -821,7 +821,9 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     int clusters = sms / 2;
     if (tiles < clusters) clusters = tiles;
     // A last wave that fills at most half of the clusters: each of its tiles becomes two of 128 columns, side by side.
-    // 8 x 512 x 4096 x 4096 (256 tiles on 74 clusters, 3.46 waves): quantizer + GEMM 68.9 us a pass whole, 67.1 split.
+    // Whole / split, us a pass of quantizer + GEMM behind an L2 flush: 4096 x 2560 x 8192 (160 tiles on 74 clusters) 95.2 / 87.0,
+    // 8 x 512 x 4096 x 4096 (256) 70.7 / 66.6, 4096 x 5120 x 8192 (320) 142.4 / 134.1, 4096 x 7168 x 4096 (448) 101.4 / 97.3,
+    // 8192 x 4864 x 8192 (608) 250.9 / 242.7; of nine such M, N at K = 1024, 4096 and 8192 none was behind.
     const int last = tiles % clusters;
     p.split_from = tiles > clusters && 2 * last <= clusters ? tiles - last : tiles;
     const int threads = gemm_threads<256, kBlockScale, true>();
@@ -1022,7 +1024,9 @@ int hkb_moe_gemm_fp8_blockscale(const void* X, const void* W, void* Y, const flo
         sa = (const float*)xsg;
     }
     GemmParams p{};
-    p.group_m = group_m_env() ? group_m_env() : 16;      // 8192 tokens, top-2 of 8 experts, N = 14336, K = 4096: 1292 us a pass, 1313 with 8
+    // 16 against 8 M blocks per group, top-2 routing, us a pass: N = 14336, K = 4096, 8 experts, 8192 tokens 1091 / 1111 and 4096
+    // tokens 581 / 592; 16 experts, N = 8192, K = 1024, 8192 tokens 269 / 275; narrower N or fewer tokens -1.3 to +0.7 %.
+    p.group_m = group_m_env() ? group_m_env() : 16;
     p.M = (int)rows; p.N = (int)N; p.K = (int)K; p.batch = 1;
     p.sa = sa; p.sb = W_scale; p.C = (__nv_bfloat16*)Y; p.gn = 128;
     p.ldc = N; p.wait_ns = kWaitLimitNs; p.skip_kblock = -1;

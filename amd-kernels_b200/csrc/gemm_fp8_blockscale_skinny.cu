@@ -20,7 +20,9 @@
 // Every K block is promoted in order with the same fused multiply-adds as in the large kernel, so the two give the same
 // bits.  Cold L2, us, large kernel / this one: 24 x 14336 x 4096 24.8 / 16.2, 32 x 28672 x 8192 53.8 / 44.7 (5.3 TB/s),
 // 16 x 57344 x 4096 75.2 / 39.5 (6.0 TB/s), 32 x 1024 x 8192 26.8 / 20.3, 8 x 4096 x 4096 16.0 / 11.3, 1 x 1024 x 1024
-// 7.9 / 6.0.  With 64 tokens the epilogue's scale reads take over (64 x 28672 x 8192 57.4 / 64.6): those stay there.
+// 7.9 / 6.0.  With multiply-add, quantizer included: 17 x 1024 x 1024 19.5 / 13.3, 17 x 4096 x 4096 27.6 / 19.5,
+// 17 x 28672 x 8192 78.9 / 62.5 (c_a and c_b loaded token by token behind the stores instead: 21.5, 27.7, 76.8).  With 64
+// tokens the epilogue's scale reads take over (64 x 28672 x 8192 57.4 / 64.6): those stay there.
 //
 // Roles: warp 0 TMA producer, warp 1 TMEM allocator + MMA issuer, warps 2-9 epilogue, warps 10-11 scale staging.  Bounded
 // waits and teardown as in gemm_fp8.cu.

@@ -687,8 +687,11 @@ int launch_prepass(const SfJob& ja, const SfJob& jb, const GatherJob& jg, cudaSt
 // reads from shared memory per K step (128 rows of A + bn rows of B) where the tiles share operands through L2, and to the
 // weight columns alone where every tile streams its own weights from HBM (`streams`: grouped calls with about one M
 // tile per expert); the width whose waves sum up to less wins.
-// M = 1000, N = 3080, K = 4224 with c_a / c_b: 19.0 us with 192 columns (136 tiles, one wave), 21.4 with 128 (200 tiles);
-// 8 experts of 8192 x 8192 with 16 rows each: 51.8 us with 128 columns (3.46 waves), 53.7 with 192 (2.32).
+// 128 / 192 columns, us a pass of quantizer + GEMM, K = 4096: 1000 x 3080 16.5 / 14.0, 128 x 20000 18.9 / 16.0, 1280 x 4096
+// 21.6 / 20.4, 256 x 8192 12.1 / 13.5, 1024 x 4096 16.8 / 19.7, 128 x 28672 19.9 / 24.3; of 20 such M, N at two K the rule took the
+// faster width each time.  Grouped, top-2 of 8, K = 4096, N = 4096: 64 tokens 21.1 / 24.5, 512 27.7 / 27.2, 700 32.3 / 32.7, 4000
+// 93.4 / 85.3; N = 14336: 400 60.8 / 61.5, 700 80.9 / 76.4, 4000 283 / 253.  Farthest off: 4000 tokens on 16 experts of
+// 2048 x 2048, 40.6 / 42.0.
 int mxfp4_tile_width(int64_t m_blks, int64_t N, int64_t batch, int sms, bool streams) {
     auto cost = [&](int bn) {
         const int64_t tiles = m_blks * ((N + bn - 1) / bn) * batch;

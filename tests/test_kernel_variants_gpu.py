@@ -1,4 +1,8 @@
 """GPU tier: the edges of single kernels and of the dispatch rules between them, against the oracle or an exact restatement."""
+import ctypes
+import os
+import threading
+
 import pytest
 import torch
 
@@ -142,6 +146,55 @@ def test_blockscale_skinny_pitched_result(hk, shape):
     assert torch.equal(out[:M, col0:col0 + N], plain)
     out[:M, col0:col0 + N] = 7.0
     assert bool((out == 7.0).all())
+
+
+@pytest.mark.parametrize("kind", ["pts", "blockscale", "mxfp4"])
+def test_decode_kernels_from_two_host_threads(hk, kind):
+    """Two shapes whose launches need different amounts of shared memory, each called from its own thread on its own stream through
+    the C ABI (ctypes lets go of the interpreter's lock): every call is accepted and gives what it gives alone."""
+    lib = ctypes.CDLL(os.path.join(os.path.dirname(hk.__file__), "..", "kernels", "libhkb200.so"))
+    i64, K = ctypes.c_int64, 1024
+    g = torch.Generator().manual_seed(1)
+    jobs = []
+    for M, N in [(16, 14336), (1, 1024)]:
+        bytes_ = lambda *s: torch.randint(0, 0x70, s, generator=g, dtype=torch.uint8).to(DEV)       # noqa: E731, B023
+        scale = lambda *s: (torch.rand(*s, generator=g) * 0.1 + 0.01).to(DEV)                        # noqa: E731, B023
+        C = [torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in range(8)]
+        if kind == "mxfp4":
+            ops, fn, mid = (bytes_(M, K // 2), bytes_(N, K // 2), bytes_(M, K // 32), bytes_(N, K // 32)), lib.hkb_gemm_mxfp4, (i64(1),)
+        elif kind == "pts":
+            ops, fn, mid = (bytes_(M, K), bytes_(N, K), scale(M), scale(N)), lib.hkb_gemm_fp8_pts, (None, i64(1))
+        else:
+            ops, fn, mid = (bytes_(M, K), bytes_(N, K), scale(M, K // 128), scale(K // 128, N // 128)), lib.hkb_gemm_fp8_blockscale, (i64(128),)
+
+        def call(c, stream, ops=ops, fn=fn, mid=mid, M=M, N=N):
+            a, b, sa, sb = (ctypes.c_void_p(t.data_ptr()) for t in ops)
+            return fn(a, b, ctypes.c_void_p(c.data_ptr()), sa, sb, *mid, i64(M), i64(N), i64(K), ctypes.c_void_p(stream.cuda_stream))
+
+        want = torch.empty_like(C[0])
+        assert call(want, torch.cuda.current_stream()) == 0
+        jobs.append((call, C, want, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    codes = [[] for _ in jobs]
+    start = threading.Barrier(len(jobs))
+
+    def work(i):
+        call, C, _, stream = jobs[i]
+        torch.cuda.set_device(0)
+        start.wait()
+        for n in range(400):
+            codes[i].append(call(C[n % len(C)], stream))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    _status_ok()
+    assert codes == [[0] * 400] * len(jobs)
+    for _, C, want, _ in jobs:
+        assert want.abs().max() > 0 and all(torch.equal(c, want) for c in C)
 
 
 def test_shim_reads_tensors_parameters_and_subclasses_alike(hk):

@@ -125,6 +125,28 @@ def test_blockscale_skinny_kernel(hk, shape):
     assert torch.equal(C, big[:M]) and torch.equal(C_ma, big_ma[:M])
 
 
+@pytest.mark.parametrize("kind,M,N", [("blockscale", 1, 128), ("blockscale", 9, 2560), ("blockscale", 32, 19072), ("blockscale", 200, 512),
+                                      ("mxfp4", 5, 2560), ("mxfp4", 64, 36000), ("mxfp4", 300, 520), ("mxfp4", 2400, 3072)])
+def test_mul_add_in_place(hk, kind, M, N):
+    """C may be c_a or c_b itself: both are read ahead of the stores, each element by the thread that then writes it."""
+    K = 256
+    g = torch.Generator().manual_seed(5)
+    if kind == "mxfp4":
+        ops = [_dev(v) for v in _mxfp4_operands(M, N, K)]
+        dispatch = hk.fused_gemm.afp4wfp4_mul_add.dispatch
+    else:
+        aq, bq, _, _ = _fp8_operands(M, N, K)
+        ops = [_dev(aq), _dev(bq), (torch.rand(M, K // 128, generator=g) * 0.1 + 0.01).to(DEV), (torch.rand(K // 128, N // 128, generator=g) * 0.1 + 0.01).to(DEV)]
+        dispatch = hk.fused_gemm.a8w8_blockscale_mul_add.dispatch
+    c_a, c_b = (torch.randn(M, N, generator=g).bfloat16().to(DEV) for _ in range(2))
+    want, in_a, in_b = torch.empty_like(c_a), c_a.clone(), c_b.clone()
+    for C, a, b in [(want, c_a, c_b), (in_a, in_a, c_b), (in_b, c_a, in_b)]:
+        dispatch(ops[0], ops[1], C, ops[2], ops[3], a, b)
+    torch.cuda.synchronize()
+    _status_ok()
+    assert torch.equal(in_a, want) and torch.equal(in_b, want) and not torch.equal(want, c_b)
+
+
 @pytest.mark.parametrize("shape", [(1, 128, 128), (17, 2560, 640), (32, 14336, 256)])
 def test_blockscale_skinny_pitched_result(hk, shape):
     """One destination with a row pitch: the column slab of a wider matrix, nothing outside it touched."""
